@@ -60,6 +60,7 @@ extern "C" int pfag_set_launch_shape(pfag_ctx *c, int coop_blocks, long update_w
     if (c->path != PFAG_PATH_FUSED) { pfag_set_error("launch shapes exist on the fused path only"); return PFAG_E_UNSUPPORTED; }
     FusedRes *r = F(c);
     r->coop_r = coop_blocks > 0 ? std::min(coop_blocks, r->coop_default) : r->coop_default;
+    r->coop_l = coop_blocks > 0 ? std::min(coop_blocks, r->coop_l_default) : r->coop_l_default;
     r->upd_warps = update_warps > 0 ? update_warps : r->upd_default;
     fused_drop_graph(r);      // the captured step holds the old grid sizes
     r->graph_state = 0;

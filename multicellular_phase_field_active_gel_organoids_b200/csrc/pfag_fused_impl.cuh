@@ -1,7 +1,7 @@
 // Fused path: the same step as the plain path (and the reference loop body,
 // main_code/run_with_active_gels.cpp:123-182), restricted to the sites that
-// can change, with no host round trip: about 18 kernels per step (9 on the
-// main stream, 9 on a side stream for the lumen/ECM work), replayed as one
+// can change, with no host round trip: about 18 kernels per step (8 on the
+// main stream, 10 on a side stream for the lumen/ECM work), replayed as one
 // CUDA graph from the second step on.
 //
 // Exactness of the restriction.  Every per-cell write of the reference step
@@ -39,6 +39,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <algorithm>
+#include <array>
 #include <climits>
 #include <cmath>
 #include <vector>
@@ -71,6 +72,20 @@ constexpr int RT_I = 8;            // reshaping tile: RT_I zone rows x the full 
 
 struct LumMaps;
 
+// launch geometry of kf_relax_cells
+struct RelaxGeom {
+    int C;          // blocks per cluster (1: a block barrier instead of the cluster's)
+    int RC;         // zone rows per block
+    int cw, g, RG;  // column warps (31 zone columns each), row groups, rows per group
+    int RGT;        // rows per group the kernel is built for (0: any, normals in shared memory)
+};
+// A sum as (units of 2^24, rest) of the loops' fixed-point unit, parts that a
+// warp adds as 32-bit integers (kf_relax_cells, FP32)
+struct RelaxUnits {
+    float f24;                    // 2^24 units as a factor on the sum of |Q - P|
+    unsigned long long thr;       // the threshold in units (2^44 .. 2^45)
+};
+
 struct FusedRes {
     void *Y1, *Y2;          // complex [Ntot][M][M]
     void *Rb;               // real [Ntot][M][M]   reaction -deg*rho + gen*P on the box
@@ -102,8 +117,13 @@ struct FusedRes {
     cudaEvent_t ev_psi, ev_area, ev_boxA, ev_lum;
     bool fork;
     int npsi;
-    int coop_r;             // co-resident block count of the persistent kernel
+    int coop_r;             // co-resident block count of the persistent cells kernel
     int coop_default;       // its value before any launch-shape setting
+    int coop_l, coop_l_default;   // the same of the persistent lumen / ECM kernel
+    bool clusters;          // the cells' loops run one cluster per cell (kf_relax_cells)
+    RelaxGeom rg;           // its geometry
+    RelaxUnits ru;          // its fixed-point sums (FP32)
+    size_t rg_smem;
     long upd_default;       // the phi update's warp budget before any launch-shape setting
     bool generic;           // box not a power of two in 16..1024: Bluestein passes (M <= 512)
     int blue_L;             // their inner power-of-two length (>= 2M-1, at least 32)
@@ -1918,7 +1938,7 @@ __global__ void kfl_normals(const real *__restrict__ lum, const real *__restrict
 constexpr int LUM_LRI = 4;
 
 // Relaxation of the lumen and ECM fields (cell_phase_functions.cpp:774-869)
-// from iteration a.it0 on, inside the persistent kernel kf_relax_loops.
+// from iteration a.it0 on, inside the persistent kernel kf_lum_loops.
 template <typename real>
 __device__ __forceinline__ void lum_loops(real *__restrict__ lum, real *__restrict__ lumn, real *__restrict__ ecm,
                                           real *__restrict__ ecmn, const real *__restrict__ Jl, const LumArgs &a,
@@ -2371,19 +2391,354 @@ __device__ __forceinline__ void centroid_rows(const real *__restrict__ phi, cons
     }
 }
 
-// The step's device-side loops in one persistent cooperative kernel: the
-// cells' reshaping from iteration ra.it0 - 1's decision on, the next step's
-// centroid sums of the reshaped cells, the lumen / ECM relaxation from
-// iteration la.it0 on, then lum <- lumn, ECM <- ECMn for the fields whose
-// loops ran here.
+// ---- reshaping of one cell by one thread-block cluster ----------------------
+// (cell_phase_functions.cpp:461-579)  The cells' relaxation loops are
+// independent of one another, so each runs on its own cluster of C blocks and
+// needs no grid barrier.  The zone's rows are split over the blocks and the
+// iterates stay in shared memory for the whole loop: a warp owns 31 zone columns x RG
+// rows (lane 0 only evaluates the face to the left of them), each face's term
+// is evaluated once and used by both its sites, and the normals of the warp's
+// faces stay in registers (RGT > 0) or are read again in every iteration,
+// mostly from L1 (RGT = 0: more rows than the registers of a block hold).  A block's first and last row also go to the
+// neighbour blocks' halo rows (distributed shared memory); one cluster
+// barrier per iteration.
+// The loop decision runs two iterations behind, so that no warp waits for the
+// sum: in iteration it the warps leave their sums of |Q - P|, in it + 1 one
+// extra warp adds them and writes the block's total into every block's table,
+// in it + 2 every warp adds the table (the same order everywhere) and, when
+// iteration it was the last, drops the iterates made since.  Three iterates
+// are kept: with it the last, phi is iterate it - 1.
+// An FP64 warp sum is ten shuffles and five FP64 additions one after another,
+// about 450 cycles, as much as the cluster barrier.  The FP32 build therefore
+// adds its threads' FP32 sums as fixed-point integers with the warp's integer
+// reduction: units of 2^-44 of the loop's threshold or finer, each sum rounded
+// to the nearest unit (a cell's total is then within 1e-12 of the threshold),
+// capped above the threshold (a NaN counts as that cap), where only the
+// comparison's outcome matters.  A thread's FP32 sum runs over the zone rows
+// 8k .. 8k + 7 of one column, as in kf_resh_first and kf_relax_loops, so the
+// three take the same decisions: the FP32 blocks and warps own whole groups of
+// eight rows.
+constexpr int RELAX_COLS = 31;
+// threads a block of kf_relax_cells may have: 128 registers each, half for the
+// FP32 form that reads the normals again
+template <typename real, int RGT> struct RelaxMax {
+    static constexpr int THREADS = sizeof(real) == 4 && RGT == 0 ? 1024 : 512;
+};
+
+// The part of a face term that its two sites share: the flux is s * inner
+// (added to one site, subtracted from the other, each as one fused
+// multiply-add like resh_update_f's).
+__device__ __forceinline__ float resh_inner_f(const ReshConst &k, float s, float pa, float pb, float ha, float hb,
+                                              float tang, float t) {
+    return fmaf(k.a4 * (pa - pb), s, fmaf(k.a16 * tang, t, -k.b4 * (ha + hb)));
+}
+
+constexpr unsigned RELAX_CAP = 1u << 26;     // 32 lanes of this stay below 2^32; the threshold is at most 2^21
+__device__ __forceinline__ unsigned long long relax_warp_total(unsigned hi, unsigned lo) {
+    const unsigned h = __reduce_add_sync(0xffffffffu, hi), l = __reduce_add_sync(0xffffffffu, lo);
+    return ((unsigned long long)h << 24) + l;
+}
+__device__ __forceinline__ unsigned long long relax_warp_total(unsigned long long v) {
+    return relax_warp_total((unsigned)min(v >> 24, (unsigned long long)RELAX_CAP), (unsigned)v & 0xffffffu);
+}
+__device__ __forceinline__ unsigned long long relax_warp_total(float f, const RelaxUnits &u) {
+    const float v = fminf(f * u.f24, (float)RELAX_CAP);       // fminf drops a NaN
+    const unsigned hi = (unsigned)v;
+    return relax_warp_total(hi, __float2uint_rn((v - (float)hi) * 16777216.0f));
+}
+
+// Block sums of (c, sx, sy) into out[0..2] (shared), which the caller zeroed
+// before a barrier; a barrier follows in the caller.
+__device__ __forceinline__ void block_counts(int c, int sx, int sy, int *out) {
+    c = __reduce_add_sync(0xffffffffu, c);
+    sx = __reduce_add_sync(0xffffffffu, sx);
+    sy = __reduce_add_sync(0xffffffffu, sy);
+    if ((threadIdx.x & 31) == 0 && c) {
+        atomicAdd(&out[0], c);
+        atomicAdd(&out[1], sx);
+        atomicAdd(&out[2], sy);
+    }
+}
+
+// One cell's centroid counts over its support rectangle outside the zone.
+template <typename real>
+__device__ __forceinline__ void outside_counts(const real *__restrict__ p, const int4 r, int zi0, int zj0, int Z,
+                                               int N, int &c, int &sx, int &sy) {
+    const int i0[4] = {r.x, zi0 + Z, zi0, zi0}, i1[4] = {zi0, r.y, zi0 + Z, zi0 + Z};
+    const int j0[4] = {r.z, r.z, r.z, zj0 + Z}, j1[4] = {r.w, r.w, zj0, r.w};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int w = j1[q] - j0[q], h = i1[q] - i0[q];
+        if (w <= 0 || h <= 0) continue;
+        for (int e = threadIdx.x; e < w * h; e += blockDim.x) {
+            const int i = i0[q] + e / w, j = j0[q] + e % w;
+            if (p[(size_t)i * N + j] > (real)0.5) { c++; sx += i; sy += j; }
+        }
+    }
+}
+
+template <typename real, int RGT>
+__global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(real *__restrict__ phi,
+                                                                      const real *__restrict__ P0,
+                                                                      const real *__restrict__ Jc,
+                                                                      const int *__restrict__ xc,
+                                                                      const int *__restrict__ yc, ReshArgs a,
+                                                                      RelaxGeom gm, RelaxUnits un,
+                                                                      const int4 *__restrict__ rect,
+                                                                      long long *__restrict__ cacc) {
+    constexpr bool F32 = sizeof(real) == 4;
+    constexpr int RR = RGT > 0 ? RGT : 1;
+    extern __shared__ double relax_sm[];
+    __shared__ int s_cnt[3], s_all[16][3];
+    // sums: FP32 fixed-point, one per warp; FP64 one per thread (RGT > 0) or warp
+    typedef typename std::conditional<F32, unsigned long long, double>::type sum_t;
+    __shared__ sum_t s_tab[2][16];
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = gm.C, rank = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = gm.cw * gm.g;   // warp nw adds the sums
+    const bool adder = warp == nw;
+    const int N = a.N, z = a.z, Z = 2 * z, W = Z + 2;
+    const int plane = (gm.RC + 2) * W;
+    const int np = RGT > 0 && !F32 ? 32 * nw : nw;                // sums an iteration leaves
+    sum_t *wsum = reinterpret_cast<sum_t *>(relax_sm);            // [2][np]
+    real *P = reinterpret_cast<real *>(wsum + 2 * np);           // [3][RC + 2][W]
+    const int r0 = rank * gm.RC, nr = min(gm.RC, Z - r0);        // this block's zone rows (nr <= 0: none)
+    real *Pup = nullptr, *Pdn = nullptr;                          // the neighbour blocks' iterates
+    sum_t *ptab = nullptr;                                        // block `lane`'s table
+    if (C > 1) {
+        if (rank > 0 && nr > 0) Pup = cl.map_shared_rank(P, rank - 1);
+        if (rank + 1 < C && r0 + gm.RC < Z) Pdn = cl.map_shared_rank(P, rank + 1);
+        if (lane < C) ptab = cl.map_shared_rank(&s_tab[0][0], lane);
+    } else if (lane == 0) {
+        ptab = &s_tab[0][0];
+    }
+    const int col = warp % gm.cw, grp = warp / gm.cw;
+    const int j = col * RELAX_COLS + lane - 1;                    // zone column; lane 0 only gives its right face
+    const bool out = lane > 0 && j < Z;
+    const int c = min(j + 1, Z), cm = max(c - 1, 0);
+    const int ra = grp * gm.RG, rb = adder ? 0 : min(ra + gm.RG, nr);
+    const ReshConst kc = resh_const(a.A, a.B);
+    const real A = (real)a.A, B = (real)a.B;
+    const int n = blockIdx.y;
+    const int zi0 = xc[n] - z, zj0 = yc[n] - z;
+    real *ph = phi + (size_t)n * N * N;
+    if (threadIdx.x < 3) s_cnt[threadIdx.x] = 0;
+    // the normals of zone rows r0 - 1 .. (W columns from the zone's left ring)
+    const real *Jx = Jc + (size_t)n * 2 * W * W + (size_t)r0 * W, *Jy = Jx + (size_t)W * W;
+    // normals of this thread's faces: xs, xt of the faces above its rows and
+    // below the last (index 0: above the first), ys, yt of the right faces;
+    // FP32 keeps the sums of the two sites' normals, FP64 the sites' own
+    real xs[RR + 1], xt[RR + 1], ys[RR], yt[RR];
+    if (nr > 0) {
+        // rows r0 - 1 .. r0 + nr of iterate 0 (ring sites, which no iteration
+        // writes, from phi) into the three buffers
+        const real *src = P0 + (size_t)n * N * N + (size_t)(zi0 + r0 - 1) * N + (zj0 - 1);
+        const real *ring = ph + (size_t)(zi0 + r0 - 1) * N + (zj0 - 1);
+        for (int r = warp; r < nr + 2; r += nw + 1) {
+            const bool edge_row = r0 + r == 0 || r0 + r == Z + 1;
+            for (int q = lane; q < W; q += 32) {
+                const bool edge = edge_row || q == 0 || q == W - 1;
+                const int o = r * W + q;
+                const real *from = (edge ? ring : src) + (size_t)r * N + q;
+                cp_async_elem(P + o, from);
+                if (edge) {
+                    cp_async_elem(P + plane + o, from);
+                    cp_async_elem(P + 2 * plane + o, from);
+                }
+            }
+        }
+        if constexpr (RGT > 0) {
+            const real *jx = Jx + ra * W + c, *jy = Jy + ra * W + c;
+            real x0 = (real)0.0, y0 = (real)0.0;
+            if (ra < rb) { x0 = jx[0]; y0 = jy[0]; }
+#pragma unroll
+            for (int k = 0; k <= RR; k++) {
+                const bool in = ra + k <= rb && ra < rb;         // row ra + k (rb: the row below the last)
+                const real x1 = in ? jx[(k + 1) * W] : (real)0.0, y1 = in ? jy[(k + 1) * W] : (real)0.0;
+                if constexpr (F32) { xs[k] = x1 + x0; xt[k] = y1 + y0; }
+                else { xs[k] = (real)0.5 * (x1 + x0); xt[k] = (real)0.5 * (y1 + y0); }
+                if (k < RR) {
+                    const real xr = in ? jx[(k + 1) * W + 1] : (real)0.0, yr = in ? jy[(k + 1) * W + 1] : (real)0.0;
+                    if constexpr (F32) { ys[k] = yr + y1; yt[k] = xr + x1; }
+                    else { ys[k] = (real)0.5 * (yr + y1); yt[k] = (real)0.5 * (xr + x1); }
+                }
+                x0 = x1; y0 = y1;
+            }
+        }
+    }
+    cp_async_wait_all();
+    if (C > 1) cl.sync(); else __syncthreads();
+    int bi = 0, it = 1, last = 0;                                 // bi: buffer of the iterate read
+    for (;; it++) {
+        if (it >= 3) {                                            // the decision after iteration it - 2
+            const int d = it - 2;
+            const sum_t mine = lane < C ? s_tab[d & 1][lane] : (sum_t)0;
+            bool below;
+            if constexpr (F32) {
+                below = relax_warp_total(mine) <= un.thr;
+            } else {
+                double rdev = mine;
+                for (int o = 8; o > 0; o >>= 1) rdev += __shfl_xor_sync(0xffffffffu, rdev, o);
+                below = __shfl_sync(0xffffffffu, rdev, 0) <= a.thr;
+            }
+            unsigned bits = 0;
+            bool stop = false;
+            if (d - 1 > a.rimax) { bits = ERRBIT_RELAX; stop = true; }
+            if (below) stop = true;
+            if (!stop && d == a.cap) { bits = ERRBIT_ITER_CAP; stop = true; }
+            if (stop) {
+                if (bits && rank == 0 && threadIdx.x == 0) atomicOr(a.err, bits);
+                last = d;
+                break;
+            }
+        }
+        const int bo = bi == 2 ? 0 : bi + 1;
+        const real *Pc = P + bi * plane;
+        real *Pn = P + bo * plane;
+        if (adder) {
+            if (it > 1) {
+                sum_t t;
+                if constexpr (F32) t = relax_warp_total(lane < np ? wsum[((it - 1) & 1) * np + lane] : 0ull);
+                else t = warp_sum_fixed(wsum + ((it - 1) & 1) * np, np);
+                if (ptab) ptab[((it - 1) & 1) * 16 + rank] = t;
+            }
+        } else {
+            double acc = 0.0;
+            float facc = 0.0f;
+            unsigned long long units = 0;
+            if (ra < rb) {
+                const real *q = Pc + ra * W;                      // smem row ra = zone row ra - 1
+                real u0l = q[cm], u0c = q[c], u0r = q[c + 1];
+                real u1l = q[W + cm], u1c = q[W + c], u1r = q[W + c + 1];
+                // the face above row ra: FP32 its normal sum and inner part, FP64 its flux
+                real sm = (real)0.0, im, x1 = (real)0.0, y1 = (real)0.0, x1r = (real)0.0, y1r = (real)0.0;
+                real fs, ft;
+                if constexpr (RGT > 0) {
+                    fs = xs[0]; ft = xt[0];
+                } else {
+                    const real *jx = Jx + ra * W + c, *jy = Jy + ra * W + c;
+                    x1 = jx[W]; y1 = jy[W]; x1r = jx[W + 1]; y1r = jy[W + 1];
+                    if constexpr (F32) { fs = x1 + jx[0]; ft = y1 + jy[0]; }
+                    else { fs = (real)0.5 * (x1 + jx[0]); ft = (real)0.5 * (y1 + jy[0]); }
+                }
+                float h1 = 0.0f;
+                if constexpr (F32) {
+                    h1 = fmaf(-u1c, u1c, u1c);
+                    sm = fs;
+                    im = resh_inner_f(kc, fs, u1c, u0c, h1, fmaf(-u0c, u0c, u0c), (u1r - u1l) + (u0r - u0l), ft);
+                } else {
+                    im = resh_flux(A, B, fs, u1c, u0c, u1r + u0r - u1l - u0l, ft);
+                }
+                const auto row = [&](int r, real ps, real pt, real ss, real st) {
+                    const real *q2 = Pc + (r + 2) * W;
+                    const real u2l = q2[cm], u2c = q2[c], u2r = q2[c + 1];
+                    real x2 = (real)0.0, y2 = (real)0.0, x2r = (real)0.0, y2r = (real)0.0;
+                    if constexpr (RGT == 0) {
+                        const real *jx2 = Jx + (r + 2) * W + c, *jy2 = Jy + (r + 2) * W + c;
+                        x2 = jx2[0]; y2 = jy2[0]; x2r = jx2[1]; y2r = jy2[1];
+                        ps = x2 + x1; pt = y2 + y1; ss = y1r + y1; st = x1r + x1;
+                        if constexpr (!F32) { ps *= (real)0.5; pt *= (real)0.5; ss *= (real)0.5; st *= (real)0.5; }
+                    }
+                    real pn;
+                    if constexpr (F32) {
+                        const float h2 = fmaf(-u2c, u2c, u2c), hr = fmaf(-u1r, u1r, u1r);
+                        const float ip = resh_inner_f(kc, ps, u2c, u1c, h2, h1, (u2r - u2l) + (u1r - u1l), pt);
+                        const float iy = resh_inner_f(kc, ss, u1r, u1c, hr, h1, (u2r - u0r) + (u2c - u0c), st);
+                        const float sl = __shfl_up_sync(0xffffffffu, ss, 1), il = __shfl_up_sync(0xffffffffu, iy, 1);
+                        const float fp = __fmul_rn(ps, ip);
+                        pn = ((r & 7) == 7) ? fmaf(ps, ip, u1c) : __fadd_rn(u1c, fp);
+                        pn = fmaf(ss, iy, pn);
+                        pn = ((r & 7) == 0) ? fmaf(-sm, im, pn) : __fsub_rn(pn, __fmul_rn(sm, im));
+                        pn = fmaf(-sl, il, pn);
+                        sm = ps; im = ip; h1 = h2;
+                    } else {
+                        const real fp = resh_flux(A, B, ps, u2c, u1c, u2r + u1r - u2l - u1l, pt);
+                        const real fy = resh_flux(A, B, ss, u1r, u1c, u2r + u2c - u0r - u0c, st);
+                        const real fl = __shfl_up_sync(0xffffffffu, fy, 1);
+                        pn = u1c;
+                        pn += fp;
+                        pn += fy;
+                        pn -= im;
+                        pn -= fl;
+                        im = fp;
+                    }
+                    if (out) {
+                        Pn[(r + 1) * W + c] = pn;
+                        if (r == 0 && Pup) Pup[bo * plane + (gm.RC + 1) * W + c] = pn;
+                        if (r == gm.RC - 1 && Pdn) Pdn[bo * plane + c] = pn;
+                        if constexpr (F32) facc += fabsf(pn - u1c);
+                        else acc += fabs((double)pn - (double)u1c) * a.scale;
+                    }
+                    u0l = u1l; u0c = u1c; u0r = u1r;
+                    u1l = u2l; u1c = u2c; u1r = u2r;
+                    if constexpr (RGT == 0) { x1 = x2; y1 = y2; x1r = x2r; y1r = y2r; }
+                };
+                if constexpr (RGT > 0) {
+#pragma unroll
+                    for (int k = 0; k < RR; k++)
+                        if (ra + k < rb) row(ra + k, xs[k + 1], xt[k + 1], ys[k], yt[k]);   // warp-uniform
+                } else {
+#pragma unroll 2
+                    for (int r = ra; r < rb; r++) {
+                        row(r, (real)0.0, (real)0.0, (real)0.0, (real)0.0);
+                        if constexpr (F32) {
+                            if (((r - ra) & 7) == 7) { units += relax_warp_total(facc, un); facc = 0.0f; }
+                        }
+                    }
+                }
+                if constexpr (F32) units += relax_warp_total(facc, un);
+            }
+            if constexpr (F32) {
+                if (lane == 0) wsum[(it & 1) * np + warp] = units;
+            } else if constexpr (RGT > 0) {
+                wsum[(it & 1) * np + threadIdx.x] = acc;
+            } else {
+                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                if (lane == 0) wsum[(it & 1) * np + warp] = acc;
+            }
+        }
+        if (C > 1) cl.sync(); else __syncthreads();
+        bi = bo;
+    }
+    // phi keeps the penultimate iterate, last - 1: the buffer written next
+    // (iterate it - 1 = last + 1 was to be read); the next step's centroid
+    // counts with it
+    int cc = 0, sx = 0, sy = 0;
+    const real *Pc = P + (bi == 2 ? 0 : bi + 1) * plane;
+    for (int r = warp; r < nr; r += nw + 1) {
+        for (int k = lane; k < Z; k += 32) {
+            const real v = Pc[(r + 1) * W + k + 1];
+            const int i = zi0 + r0 + r, jj = zj0 + k;
+            ph[(size_t)i * N + jj] = v;
+            if (v > (real)0.5) { cc++; sx += i; sy += jj; }
+        }
+    }
+    if (rank == 0) {
+        outside_counts<real>(ph, rect[n], zi0, zj0, Z, N, cc, sx, sy);
+        if (threadIdx.x == 0) { a.K[n] = last; a.done[n] = last; }
+    }
+    block_counts(cc, sx, sy, s_cnt);
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        if (C > 1) cl.map_shared_rank(&s_all[0][0], 0)[rank * 3 + threadIdx.x] = s_cnt[threadIdx.x];
+        else s_all[0][threadIdx.x] = s_cnt[threadIdx.x];
+    }
+    if (C > 1) cl.sync(); else __syncthreads();
+    if (rank == 0 && threadIdx.x < 3) {
+        long long t = 0;
+        for (int k = 0; k < C; k++) t += s_all[k][threadIdx.x];
+        cacc[3 * n + threadIdx.x] = t;
+    }
+}
+
+// The same loops for zones whose cluster does not hold the cell in shared
+// memory: one persistent cooperative kernel for all cells, from iteration
+// ra.it0 - 1's decision on, then the next step's centroid sums.
 template <typename real, int RB>
 __global__ void __launch_bounds__(RESH_MAX_THREADS, 2) kf_relax_loops(real *__restrict__ phi, real *__restrict__ phin,
                                                                     real *__restrict__ T, const real *__restrict__ Jc,
                                                                     const int *__restrict__ xc,
                                                                     const int *__restrict__ yc, ReshArgs ra,
-                                                                    real *__restrict__ lum, real *__restrict__ lumn,
-                                                                    real *__restrict__ ecm, real *__restrict__ ecmn,
-                                                                    const real *__restrict__ Jl, LumArgs la,
                                                                     const int4 *__restrict__ rect,
                                                                     long long *__restrict__ cacc) {
     cg::grid_group grid = cg::this_grid();
@@ -2392,6 +2747,16 @@ __global__ void __launch_bounds__(RESH_MAX_THREADS, 2) kf_relax_loops(real *__re
         for (int k = threadIdx.x; k < 3 * ra.Ntot; k += blockDim.x) cacc[k] = 0;
     resh_loops<real, RB>(phi, phin, T, Jc, xc, yc, ra, wacc, grid);   // ends with a grid barrier
     centroid_rows<real>(phi, rect, ra.N, ra.Ntot, cacc);
+}
+
+// The lumen / ECM relaxation from iteration la.it0 on (cooperative; returns at
+// once when both loops have stopped before), then lum <- lumn, ECM <- ECMn for
+// the fields whose loops ran here.
+template <typename real>
+__global__ void __launch_bounds__(FT, 2) kf_lum_loops(real *__restrict__ lum, real *__restrict__ lumn,
+                                                      real *__restrict__ ecm, real *__restrict__ ecmn,
+                                                      const real *__restrict__ Jl, LumArgs la) {
+    cg::grid_group grid = cg::this_grid();
     lum_loops<real>(lum, lumn, ecm, ecmn, Jl, la, grid);
     lum_copy_fields<real>(lum, lumn, ecm, ecmn, la.K, la.done, la.N, la.it0, INT_MAX,
                           (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
@@ -2582,9 +2947,12 @@ struct Fused {
             // tiles): a small organoid's persistent kernel leaves the rest of the
             // GPU to other contexts (sweep members)
             const long strips = (long)c->Ntot * r->tpc;
-            const long tiles = (long)((c->N + LUM_LRI - 1) / LUM_LRI) * ((c->N + r->resh_threads - 1) / r->resh_threads);
-            r->coop_r = (int)std::max(1L, std::min((long)r->coop_r, std::max(strips, tiles)));
+            r->coop_r = (int)std::max(1L, std::min((long)r->coop_r, strips));
+            const long tiles = (long)((c->N + LUM_LRI - 1) / LUM_LRI) * ((c->N + FT - 1) / FT);
+            PFAG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kf_lum_loops<real>, FT, 0));
+            r->coop_l = (int)std::max(1L, std::min((long)nsm * std::min(std::max(per, 1), 8), tiles));
         }
+        PFAG_TRY(choose_clusters(nsm));
         r->ntl = ((c->N + LRB - 1) / LRB) * ((c->N + FT - 1) / FT);
         r->lum_tile = (size_t)3 * (LRB + 2) * (FT + 2) * sizeof(real);
         PFAG_TRY(smem_at_least((const void *)kl_relax<real>, r->lum_tile));
@@ -2599,8 +2967,142 @@ struct Fused {
             r->upd_warps = (long)nsm * std::max(per, 1) * (UPD_THREADS / 32);
         }
         r->coop_default = r->coop_r;
+        r->coop_l_default = r->coop_l;
         r->upd_default = r->upd_warps;
         return PFAG_OK;
+    }
+
+    // Geometry of kf_relax_cells for zones of Z x Z sites: rows split over at
+    // most C blocks, 31 columns a warp, at most g row groups, one more warp for
+    // the sums.  FP32: whole groups of eight rows per block and per warp.
+    bool relax_geom(int C, int g, RelaxGeom &gm, size_t &smem) const {
+        constexpr bool F32 = sizeof(real) == 4;
+        constexpr int U = F32 ? 8 : 1;
+        const int Z = 2 * c->zone;
+        gm.RC = U * ((Z + C * U - 1) / (C * U));
+        gm.C = (Z + gm.RC - 1) / gm.RC;
+        gm.cw = (Z + RELAX_COLS - 1) / RELAX_COLS;
+        // the normals in registers when a warp has few enough rows
+        int maxw = RelaxMax<real, 8>::THREADS / 32 - 1;
+        for (int pass = 0; pass < 2; pass++) {
+            gm.g = std::min({g, maxw / gm.cw, gm.RC / U});
+            if (gm.g >= 1) {
+                gm.RG = U * ((gm.RC / U + gm.g - 1) / gm.g);
+                gm.g = (gm.RC + gm.RG - 1) / gm.RG;
+                gm.RGT = F32 ? (gm.RG == 8 ? 8 : 0) : (gm.RG <= 4 ? gm.RG : 0);
+                if (gm.RGT > 0 || pass == 1) break;
+            }
+            maxw = RelaxMax<real, 0>::THREADS / 32 - 1;
+        }
+        if (gm.g < 1) return false;
+        if (gm.RGT == 8 && 32 * (gm.cw * gm.g + 1) > RelaxMax<real, 8>::THREADS) gm.RGT = 0;
+        const int nw = gm.cw * gm.g;
+        smem = (size_t)2 * (gm.RGT && !F32 ? 32 * nw : nw) * sizeof(double) +
+               (size_t)3 * (gm.RC + 2) * (Z + 2) * sizeof(real);
+        return smem <= 226 * 1024;
+    }
+    typedef void (*relax_fn)(real *, const real *, const real *, const int *, const int *, ReshArgs, RelaxGeom,
+                             RelaxUnits, const int4 *, long long *);
+    static relax_fn relax_kernel(int RGT) {
+        if constexpr (sizeof(real) == 4) {
+            return RGT == 8 ? kf_relax_cells<real, 8> : kf_relax_cells<real, 0>;
+        } else {
+            switch (RGT) {
+            case 1: return kf_relax_cells<real, 1>;
+            case 2: return kf_relax_cells<real, 2>;
+            case 3: return kf_relax_cells<real, 3>;
+            case 4: return kf_relax_cells<real, 4>;
+            default: return kf_relax_cells<real, 0>;
+            }
+        }
+    }
+    // the fixed-point unit of FP32 sums of |Q - P|: a power of two that makes the
+    // loop's threshold 2^44 .. 2^45 units; false when the threshold is no
+    // positive number of usual size
+    bool relax_units(RelaxUnits &u) const {
+        const double t = c->dp.thr_cells / (c->dp.dx * c->dp.dx / (double)c->dp.Ncur);
+        if (!(t > 1e-18 && t < 1e18)) return false;
+        const int e = 44 - std::ilogb(t);
+        u.f24 = (float)std::ldexp(1.0, e - 24);
+        u.thr = (unsigned long long)std::ldexp(t, e);
+        return true;
+    }
+    // whether the GPU holds every cell's cluster of this geometry at once; the
+    // query for clusters takes milliseconds: only where the blocks alone fit, and
+    // once per geometry (an entry per zone size and block shape of the process)
+    int relax_resident(const RelaxGeom &gm, size_t smem, int nsm, bool *fits) const {
+        const void *fn = (const void *)relax_kernel(gm.RGT);
+        *fits = false;
+        int per = 0, ncl = 0;
+        PFAG_TRY(smem_at_least(fn, smem));
+        PFAG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 32 * (gm.cw * gm.g + 1), smem));
+        if ((long)nsm * per < (long)c->Ntot * gm.C) return PFAG_OK;
+        if (gm.C > 8) PFAG_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        static std::mutex mu;
+        static std::map<std::array<long, 5>, int> known;
+        int dev = 0;
+        PFAG_CUDA_CHECK(cudaGetDevice(&dev));
+        const std::array<long, 5> key = {dev, (long)fn, gm.C, gm.cw * gm.g, (long)smem};
+        std::lock_guard<std::mutex> lock(mu);
+        const auto hit = known.find(key);
+        if (hit != known.end()) {
+            ncl = hit->second;
+        } else {
+            cudaLaunchAttribute attr[1];
+            const cudaLaunchConfig_t cfg = relax_config(gm, smem, attr, nullptr);
+            if (cudaOccupancyMaxActiveClusters(&ncl, fn, &cfg) != cudaSuccess) {
+                (void)cudaGetLastError();
+                ncl = 0;
+            }
+            known[key] = ncl;
+        }
+        *fits = ncl >= c->Ntot;
+        return PFAG_OK;
+    }
+    // The cluster size: the barrier costs about the same from 2 to 16 blocks, so
+    // the more blocks share a cell, the shorter its iteration (FP32, 7 cells of
+    // 130 x 130, 18 iterations: 34 us with 16 blocks, 46 with 8, 70 with 4; the
+    // persistent kernel 121), as long as every cell's cluster (of 8 to 16 blocks)
+    // is resident at once.  Otherwise the cells queue for the clusters: 64 cells
+    // of 258 x 258 at 2 to 3 iterations took 437 us a step against 356 with
+    // iteration 1 at full occupancy and the persistent kernel, which organoids
+    // with that many cells keep.  Within a size the most row groups that stay
+    // resident.
+    int choose_clusters(int nsm) {
+        r->clusters = false;
+        if (sizeof(real) == 4 && !relax_units(r->ru)) return PFAG_OK;
+        for (int C = 16; C >= 8; C /= 2) {
+            int tried = 0;
+            for (int g = 32; g >= 1; g--) {
+                RelaxGeom gm{};
+                size_t smem = 0;
+                bool fits = false;
+                if (!relax_geom(C, g, gm, smem) || gm.g == tried) continue;   // gm.g <= g: the next form
+                tried = gm.g;
+                PFAG_TRY(relax_resident(gm, smem, nsm, &fits));
+                if (fits) {
+                    r->rg = gm;
+                    r->rg_smem = smem;
+                    r->clusters = true;
+                    return PFAG_OK;
+                }
+            }
+        }
+        return PFAG_OK;
+    }
+    cudaLaunchConfig_t relax_config(const RelaxGeom &gm, size_t smem, cudaLaunchAttribute *attr, cudaStream_t s) const {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(gm.C, c->Ntot);
+        cfg.blockDim = dim3(32 * (gm.cw * gm.g + 1));
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = gm.C;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        return cfg;
     }
 
     int alloc() {
@@ -2636,7 +3138,7 @@ struct Fused {
         }
         PFAG_CUDA_CHECK(cudaMalloc(&r->part_r, sizeof(double) * (size_t)c->Ntot * std::max(r->tpc, r->coop_r)));
         PFAG_CUDA_CHECK(cudaMalloc(&r->part_e, sizeof(double) * r->npsi));
-        PFAG_CUDA_CHECK(cudaMalloc(&r->part_l, sizeof(double) * 2 * r->coop_r));
+        PFAG_CUDA_CHECK(cudaMalloc(&r->part_l, sizeof(double) * 2 * r->coop_l));
         if (sizeof(real) == 4 && c->N % 4 == 0 && c->N >= LT_W) {
             // TMA-staged lumen / ECM iterations: the maps hold the addresses of
             // this context's lum, lumn, ECM, ECMn and of the normals Jl, so
@@ -2746,7 +3248,7 @@ struct Fused {
         cudaStream_t s = c->stream;
         const int N = c->N, Nt = c->Ntot, M = c->M, z = c->zone;
         const DevParams &d = c->dp;
-        // 1-2. centroids (from the sums the previous step's persistent kernel,
+        // 1-2. centroids (from the sums the previous step's last cell kernel,
         //    or the upload, left over B_n), hfunc on the zones, psi, area
         //    partials, h(lum), h(ECM), sum_ecm partials
         const int tiles = (N + 31) / 32, tiles_r = (N + PT_R - 1) / PT_R;
@@ -2766,9 +3268,10 @@ struct Fused {
         //    (cell_phase_functions.cpp:372-444, :722-771), which need only psi,
         //    h(lum) and h(ECM): on the side stream beside pass A, the phi
         //    update and the rest of the spectral solve.  The relaxation (6)
-        //    rewrites lum and ECM, so it waits for pass A, which reads them.  No
-        //    cooperative kernel runs beside the side stream: the main stream
-        //    joins it before the persistent kernel.
+        //    rewrites lum and ECM, so it waits for pass A, which reads them.  The
+        //    side stream's cooperative kernel returns at once unless a field still
+        //    moves, and the kernels beside it wait for nothing of its; the other
+        //    cooperative kernel (kf_relax_loops) is launched after the join.
         const bool fork = !pfag_prof_on(c);
         cudaStream_t s2 = fork ? r->side : s;
         r->fork = fork;
@@ -2847,7 +3350,6 @@ struct Fused {
         //    full-occupancy kernels on the side stream once pass A has read lum
         //    and ECM, and lum <- lumn, ECM <- ECMn for the fields that stopped
         //    there; the rest (if a field still moves) in the persistent kernel
-        //    after the join below
         if (fork) PFAG_CUDA_CHECK(cudaStreamWaitEvent(s2, r->ev_boxA, 0));
         for (int it = 1; it <= LUM_REGULAR; it++) {
             if constexpr (sizeof(real) == 4) {
@@ -2874,10 +3376,19 @@ struct Fused {
         kl_copy<real><<<296, FT, 0, s2>>>(R(c->lum), R(c->lumn), R(c->ecm), R(c->ecmn), r->lK, r->ldone, N,
                                           LUM_REGULAR);
         PFAG_LAUNCHED(c);
+        la.it0 = LUM_REGULAR + 1;
+        {
+            real *b0 = R(c->lum), *b1 = R(c->lumn), *b2 = R(c->ecm), *b3 = R(c->ecmn);
+            const real *b4 = R(r->Jl);
+            void *args[] = {&b0, &b1, &b2, &b3, (void *)&b4, &la};
+            pfag_prof_begin(c, "kf_lum_loops");
+            PFAG_TRY(launch_coop_t((const void *)kf_lum_loops<real>, &r->coop_l, FT, args, 0, s2));
+            PFAG_LAUNCHED(c);
+        }
         if (fork) PFAG_CUDA_CHECK(cudaEventRecord(r->ev_lum, s2));
-        // 7. reshaping of the cells: iteration 1 at full occupancy, then the
-        //    persistent kernel (its decision, iterations 2.., and the lumen /
-        //    ECM iterations beyond LUM_REGULAR)
+        // 7. reshaping of the cells: a cluster per cell; where not every cell's
+        //    cluster is resident, iteration 1 at full occupancy and the persistent
+        //    kernel, after the join
         {
             ReshArgs ra{};
             ra.N = N; ra.z = z; ra.Ntot = Nt; ra.tpc = r->tpc;
@@ -2885,27 +3396,35 @@ struct Fused {
             ra.A = d.A_resh; ra.B = d.B_resh; ra.scale = d.dx * d.dx / (double)d.Ncur; ra.thr = d.thr_cells;
             ra.K = r->cK; ra.done = r->cdone; ra.cnt = r->ccnt; ra.part = r->part_r; ra.err = c->d_err;
             ra.it0 = 2;
-            la.it0 = LUM_REGULAR + 1;
             real *T = R(c->rhon);          // the fused path keeps rho in place: rhon is the reshaping scratch
-            const dim3 gs(r->tpc, Nt);
-            pfag_prof_begin(c, "kf_resh_first");
-            kf_resh_first<real, RESH_RB><<<gs, r->resh_threads, r->resh_tile, s>>>(R(c->phin), T, R(c->phi), R(r->Jc),
-                                                                                    c->d_xc, c->d_yc, ra);
-            PFAG_LAUNCHED(c);
-            real *a0 = R(c->phi), *a1 = R(c->phin), *a2 = T;
-            const real *a3 = R(r->Jc);
-            const int *a4 = c->d_xc, *a5 = c->d_yc;
-            real *b0 = R(c->lum), *b1 = R(c->lumn), *b2 = R(c->ecm), *b3 = R(c->ecmn);
-            const real *b4 = R(r->Jl);
-            const int4 *c0 = r->rect;
-            long long *c1 = c->d_cacc;
-            void *args[] = {&a0, &a1, &a2, (void *)&a3, (void *)&a4, (void *)&a5, &ra,
-                            &b0, &b1, &b2, &b3, (void *)&b4, &la, (void *)&c0, &c1};
+            if (r->clusters) {
+                cudaLaunchAttribute attr[1];
+                const cudaLaunchConfig_t cfg = relax_config(r->rg, r->rg_smem, attr, s);
+                pfag_prof_begin(c, "kf_relax_cells");
+                PFAG_CUDA_CHECK(cudaLaunchKernelEx(&cfg, relax_kernel(r->rg.RGT), R(c->phi), (const real *)R(c->phin),
+                                                   (const real *)R(r->Jc), (const int *)c->d_xc, (const int *)c->d_yc,
+                                                   ra, r->rg, r->ru, (const int4 *)r->rect, c->d_cacc));
+                PFAG_LAUNCHED(c);
+            } else {
+                const dim3 gs(r->tpc, Nt);
+                pfag_prof_begin(c, "kf_resh_first");
+                kf_resh_first<real, RESH_RB><<<gs, r->resh_threads, r->resh_tile, s>>>(
+                    R(c->phin), T, R(c->phi), R(r->Jc), c->d_xc, c->d_yc, ra);
+                PFAG_LAUNCHED(c);
+            }
             if (fork) PFAG_CUDA_CHECK(cudaStreamWaitEvent(s, r->ev_lum, 0));   // join the side stream
-            pfag_prof_begin(c, "kf_relax_loops");
-            PFAG_TRY(launch_coop_t((const void *)kf_relax_loops<real, RESH_RB>, &r->coop_r, r->resh_threads, args,
-                                   r->resh_smem, s));
-            PFAG_LAUNCHED(c);
+            if (!r->clusters) {
+                real *a0 = R(c->phi), *a1 = R(c->phin), *a2 = T;
+                const real *a3 = R(r->Jc);
+                const int *a4 = c->d_xc, *a5 = c->d_yc;
+                const int4 *c0 = r->rect;
+                long long *c1 = c->d_cacc;
+                void *args[] = {&a0, &a1, &a2, (void *)&a3, (void *)&a4, (void *)&a5, &ra, (void *)&c0, &c1};
+                pfag_prof_begin(c, "kf_relax_loops");
+                PFAG_TRY(launch_coop_t((const void *)kf_relax_loops<real, RESH_RB>, &r->coop_r, r->resh_threads, args,
+                                       r->resh_smem, s));
+                PFAG_LAUNCHED(c);
+            }
         }
         // 8. periodic ghost ring of rho (boundary_conditions_cells(rhon),
         //    rho_functions.cpp:469).  Its sources, rows and columns 1 and N-2,

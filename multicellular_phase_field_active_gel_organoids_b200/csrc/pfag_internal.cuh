@@ -167,12 +167,16 @@ __device__ __forceinline__ real lap9(real c, real ip, real im, real jp, real jm,
 // One face term of the reshaping flux (cell_phase_functions.cpp:511-547, :802-838):
 // 0.5*(Jn_a+Jn_b) * ( A*(pa-pb)*0.5*(Jn_a+Jn_b) + A*0.25*tang*0.5*(Jt_a+Jt_b)
 //                     - B*0.5*(pa*(1-pa) + pb*(1-pb)) )
+// resh_flux takes the two means jn = 0.5*(Jn_a+Jn_b), jt = 0.5*(Jt_a+Jt_b).
+template <typename real>
+__device__ __forceinline__ real resh_flux(real A, real B, real jn, real pa, real pb, real tang, real jt) {
+    return jn * (A * (pa - pb) * jn + A * (real)0.25 * tang * jt -
+                 B * (real)0.5 * (pa * ((real)1.0 - pa) + pb * ((real)1.0 - pb)));
+}
 template <typename real>
 __device__ __forceinline__ real resh_face(real A, real B, real jn_a, real jn_b, real pa, real pb,
                                           real tang, real jt_a, real jt_b) {
-    real jn = (real)0.5 * (jn_a + jn_b);
-    return jn * (A * (pa - pb) * jn + A * (real)0.25 * tang * ((real)0.5 * (jt_a + jt_b)) -
-                 B * (real)0.5 * (pa * ((real)1.0 - pa) + pb * ((real)1.0 - pb)));
+    return resh_flux(A, B, (real)0.5 * (jn_a + jn_b), pa, pb, tang, (real)0.5 * (jt_a + jt_b));
 }
 
 // Full reshaping increment at one site given the 3x3 neighbourhood of the
