@@ -7,18 +7,14 @@ int pfag_fused_alloc_f64(pfag_ctx *c);
 int pfag_fused_alloc_f32(pfag_ctx *c);
 int pfag_fused_upload_f64(pfag_ctx *c);
 int pfag_fused_upload_f32(pfag_ctx *c);
-int pfag_fused_step_f64(pfag_ctx *c, bool sync_host);
-int pfag_fused_step_f32(pfag_ctx *c, bool sync_host);
-int pfag_fused_stats_f64(pfag_ctx *c);
-int pfag_fused_stats_f32(pfag_ctx *c);
+int pfag_fused_step_f64(pfag_ctx *c);
+int pfag_fused_step_f32(pfag_ctx *c);
 int pfag_fused_recentre_f64(pfag_ctx *c);
 int pfag_fused_recentre_f32(pfag_ctx *c);
-int pfag_fused_step_part_f64(pfag_ctx *c, int part, bool sync_host);
-int pfag_fused_step_part_f32(pfag_ctx *c, int part, bool sync_host);
+int pfag_fused_step_part_f64(pfag_ctx *c, int part);
+int pfag_fused_step_part_f32(pfag_ctx *c, int part);
 
-int pfag_fused_stats(pfag_ctx *c) {
-    return c->prec == 64 ? pfag_fused_stats_f64(c) : pfag_fused_stats_f32(c);
-}
+const int *pfag_fused_counters(pfag_ctx *c) { return F(c)->cK; }
 
 int pfag_fused_recentre(pfag_ctx *c) {
     return c->prec == 64 ? pfag_fused_recentre_f64(c) : pfag_fused_recentre_f32(c);
@@ -50,8 +46,8 @@ int pfag_fused_upload_hook(pfag_ctx *c) {
     return c->prec == 64 ? pfag_fused_upload_f64(c) : pfag_fused_upload_f32(c);
 }
 
-int pfag_fused_step(pfag_ctx *c, int, bool sync_host) {
-    return c->prec == 64 ? pfag_fused_step_f64(c, sync_host) : pfag_fused_step_f32(c, sync_host);
+int pfag_fused_step(pfag_ctx *c, int) {
+    return c->prec == 64 ? pfag_fused_step_f64(c) : pfag_fused_step_f32(c);
 }
 
 // ---- launch shapes (the autotuner's knobs) ---------------------------------
@@ -179,7 +175,7 @@ extern "C" int pfag_batch_step_async(pfag_batch *b, int it0, int nsteps) {
         if (ready) break;
         for (pfag_ctx *c : b->m) {
             const long l0 = c->launches;
-            PFAG_TRY(pfag_fused_step(c, it0 + k, false));
+            PFAG_TRY(pfag_fused_step(c, it0 + k));
             b->launches += c->launches - l0;
         }
     }
@@ -203,13 +199,10 @@ extern "C" int pfag_batch_step_async(pfag_batch *b, int it0, int nsteps) {
 
 extern "C" int pfag_batch_sync(pfag_batch *b) {
     if (!b) { pfag_set_error("null batch"); return PFAG_E_ARG; }
+    // every member's report enqueued before the first wait
+    for (pfag_ctx *c : b->m) PFAG_TRY(pfag_report(c));
     PFAG_CUDA_CHECK(cudaStreamSynchronize(b->stream));
-    for (pfag_ctx *c : b->m) {
-        PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
-        PFAG_TRY(pfag_check_device_error(c));
-        PFAG_TRY(c->prec == 64 ? pfag_fused_stats_f64(c) : pfag_fused_stats_f32(c));
-        PFAG_TRY(pfag_fetch_observables(c));
-    }
+    for (pfag_ctx *c : b->m) PFAG_TRY(pfag_finish(c, false));
     return PFAG_OK;
 }
 
@@ -249,7 +242,7 @@ static int step_part(pfag_ctx *c, int part) {
     if (!c) { pfag_set_error("null ctx"); return PFAG_E_ARG; }
     if (c->path != PFAG_PATH_FUSED) { pfag_set_error("the split step runs on the fused path"); return PFAG_E_UNSUPPORTED; }
     if (part == 1) c->launches = 0;
-    return c->prec == 64 ? pfag_fused_step_part_f64(c, part, false) : pfag_fused_step_part_f32(c, part, false);
+    return c->prec == 64 ? pfag_fused_step_part_f64(c, part) : pfag_fused_step_part_f32(c, part);
 }
 extern "C" int pfag_step_head(pfag_ctx *c, int) { return step_part(c, 1); }
 extern "C" int pfag_step_tail(pfag_ctx *c, int) { return step_part(c, 2); }

@@ -3599,35 +3599,10 @@ struct Fused {
         PFAG_CUDA_CHECK(cudaGetLastError());
         return PFAG_OK;
     }
-
-    int stats() {
-        const int Nt = c->Ntot;
-        if (std::getenv("PFAG_DEBUG_COOP")) {
-            cudaFuncAttributes fr{};
-            cudaFuncGetAttributes(&fr, (const void *)kf_relax_loops<real, RESH_RB>);
-            std::fprintf(stderr, "pfag coop: relaxation loops %d blocks x %d threads (%d regs)\n", r->coop_r,
-                         r->resh_threads, fr.numRegs);
-        }
-        std::vector<int> h(3 * Nt + 8);
-        PFAG_CUDA_CHECK(cudaMemcpyAsync(h.data(), r->cK, sizeof(int) * (3 * Nt + 8), cudaMemcpyDeviceToHost, c->stream));
-        PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
-        int mx = 0, sm = 0;
-        for (int n = 0; n < Nt; n++) {
-            c->h_iflags[4 * Nt + n] = h[n];
-            mx = std::max(mx, h[n]);
-            sm += h[n];
-        }
-        c->stats.cell_iters_max = mx;
-        c->stats.cell_iters_sum = sm;
-        c->stats.lum_iters = h[3 * Nt + 0];
-        c->stats.ecm_iters = h[3 * Nt + 1];
-        return PFAG_OK;
-    }
 };
 
 // Entry points instantiated once per precision (pfag_fused_f64.cu, pfag_fused_f32.cu).
 template <typename real> int fused_alloc_t(pfag_ctx *c) { return Fused<real>(c).alloc(); }
-template <typename real> int fused_stats_t(pfag_ctx *c) { return Fused<real>(c).stats(); }
 template <typename real> int fused_recentre_t(pfag_ctx *c) { return Fused<real>(c).recentre(); }
 template <typename real> int fused_upload_t(pfag_ctx *c) { return Fused<real>(c).upload_hook(); }
 inline void fused_drop_graph(FusedRes *r) {
@@ -3643,7 +3618,7 @@ inline void fused_drop_graph(FusedRes *r) {
 // One part of a step split at psi (part 1: head, 2: tail), graph-captured
 // like the whole step once an eager step has run: the head after the first
 // eager head-and-tail, the tail likewise.
-template <typename real> int fused_step_part_t(pfag_ctx *c, int part, bool sync_host) {
+template <typename real> int fused_step_part_t(pfag_ctx *c, int part) {
     FusedRes *r = F(c);
     if ((part == 1) == r->head_pending) {
         pfag_set_error(part == 1 ? "step head enqueued twice without its tail" : "step tail without its head");
@@ -3688,10 +3663,6 @@ template <typename real> int fused_step_part_t(pfag_ctx *c, int part, bool sync_
         }
     }
     r->head_pending = part == 1;
-    if (sync_host && part == 2) {
-        PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
-        return Fused<real>(c).stats();
-    }
     return PFAG_OK;
 }
 
@@ -3700,7 +3671,7 @@ template <typename real> int fused_step_part_t(pfag_ctx *c, int part, bool sync_
 // into a CUDA graph that every later step replays with one launch.  Profiling,
 // debug capture and PFAG_NO_GRAPH keep the eager path; a failed capture falls
 // back to it for good.
-template <typename real> int fused_step_t(pfag_ctx *c, bool sync_host) {
+template <typename real> int fused_step_t(pfag_ctx *c) {
     FusedRes *r = F(c);
     if (r->head_pending) { pfag_set_error("a step head is waiting for its tail"); return PFAG_E_ARG; }
     const bool graphable = !pfag_prof_on(c) && !c->debug && !std::getenv("PFAG_NO_GRAPH");
@@ -3739,10 +3710,6 @@ template <typename real> int fused_step_t(pfag_ctx *c, bool sync_host) {
         if (rc != PFAG_OK) return rc;
         r->eager_steps++;
         r->ring_pending = false;
-    }
-    if (sync_host) {
-        PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
-        rc = Fused<real>(c).stats();
     }
     return rc;
 }

@@ -104,6 +104,7 @@ struct pfag_ctx {
     int *h_iflags;        // pinned
     double *h_scal;       // pinned
     unsigned *h_err;      // pinned
+    void *h_rep;          // pinned, mapped: what a synchronising call reads back (pfag_finish)
     pfag_stats stats;
     long launches;
     int debug;
@@ -132,11 +133,13 @@ int pfag_plain_generate(pfag_ctx *ctx, double rho0, double tol, int make_fields)
 int pfag_fused_alloc(pfag_ctx *ctx);
 void pfag_fused_free(pfag_ctx *ctx);
 int pfag_fused_upload_hook(pfag_ctx *ctx);
-int pfag_fused_step(pfag_ctx *ctx, int it, bool sync_host);
+int pfag_fused_step(pfag_ctx *ctx, int it);
 int pfag_check_device_error(pfag_ctx *ctx);
+int pfag_report(pfag_ctx *ctx);
+int pfag_finish(pfag_ctx *ctx, bool stats_first);
 int pfag_after_upload(pfag_ctx *ctx);
 int pfag_fused_recentre(pfag_ctx *ctx);
-int pfag_fused_stats(pfag_ctx *c);        // reshaping iteration counts of the last step into c->stats
+const int *pfag_fused_counters(pfag_ctx *c);   // device: per-cell iteration counts [Ntot], ..., lumen's and ECM's at 3 Ntot
 int pfag_fetch_observables(pfag_ctx *ctx);
 
 // ---------------------------------------------------------------------------
