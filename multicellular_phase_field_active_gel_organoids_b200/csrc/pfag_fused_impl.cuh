@@ -116,6 +116,10 @@ struct FusedRes {
     cudaStream_t side;
     cudaEvent_t ev_psi, ev_area, ev_boxA, ev_lum;
     bool fork;
+    // the spectral passes beside the phi update and the cells' loops (split)
+    cudaStream_t spec;
+    cudaEvent_t ev_upd, ev_spec;
+    bool split;             // this organoid's steps run them so
     int npsi;
     int coop_r;             // co-resident block count of the persistent cells kernel
     int coop_default;       // its value before any launch-shape setting
@@ -2414,15 +2418,20 @@ __device__ __forceinline__ void centroid_rows(const real *__restrict__ phi, cons
 // reduction: units of 2^-44 of the loop's threshold or finer, each sum rounded
 // to the nearest unit (a cell's total is then within 1e-12 of the threshold),
 // capped above the threshold (a NaN counts as that cap), where only the
-// comparison's outcome matters.  A thread's FP32 sum runs over the zone rows
-// 8k .. 8k + 7 of one column, as in kf_resh_first and kf_relax_loops, so the
-// three take the same decisions: the FP32 blocks and warps own whole groups of
-// eight rows.
+// comparison's outcome matters.  An FP32 sum runs over the zone rows 8k ..
+// 8k + 7 of one column, as in kf_resh_first and kf_relax_loops, so the three
+// take the same decisions: the FP32 blocks own whole groups of eight rows.
+// The first warp of a group leaves its rows' sum, the others (4 or 2 rows a
+// warp: shorter chains and more warps to hide them) their values, and the extra
+// warp adds them in row order.  That pays in blocks of one group (45 iterations
+// of 3 cells of 34 x 34: 62 us a step with 2 rows a warp, 66 with 4, 79 with 8);
+// with two groups the extra warp is the longest (26 iterations of 130 x 130:
+// 94 with 4, 90 with 8).
 constexpr int RELAX_COLS = 31;
-// threads a block of kf_relax_cells may have: 128 registers each, half for the
-// FP32 form that reads the normals again
+// threads a block of kf_relax_cells may have: 128 registers each, fewer for the
+// FP32 forms of few rows and for the one that reads the normals again
 template <typename real, int RGT> struct RelaxMax {
-    static constexpr int THREADS = sizeof(real) == 4 && RGT == 0 ? 1024 : 512;
+    static constexpr int THREADS = sizeof(real) == 8 || RGT == 8 ? 512 : RGT == 4 ? 704 : 1024;
 };
 
 // The part of a face term that its two sites share: the flux is s * inner
@@ -2441,10 +2450,15 @@ __device__ __forceinline__ unsigned long long relax_warp_total(unsigned hi, unsi
 __device__ __forceinline__ unsigned long long relax_warp_total(unsigned long long v) {
     return relax_warp_total((unsigned)min(v >> 24, (unsigned long long)RELAX_CAP), (unsigned)v & 0xffffffu);
 }
-__device__ __forceinline__ unsigned long long relax_warp_total(float f, const RelaxUnits &u) {
+__device__ __forceinline__ void relax_units_of(float f, const RelaxUnits &u, unsigned &hi, unsigned &lo) {
     const float v = fminf(f * u.f24, (float)RELAX_CAP);       // fminf drops a NaN
-    const unsigned hi = (unsigned)v;
-    return relax_warp_total(hi, __float2uint_rn((v - (float)hi) * 16777216.0f));
+    hi = (unsigned)v;
+    lo = __float2uint_rn((v - (float)hi) * 16777216.0f);
+}
+__device__ __forceinline__ unsigned long long relax_warp_total(float f, const RelaxUnits &u) {
+    unsigned hi, lo;
+    relax_units_of(f, u, hi, lo);
+    return relax_warp_total(hi, lo);
 }
 
 // Block sums of (c, sx, sy) into out[0..2] (shared), which the caller zeroed
@@ -2502,6 +2516,10 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
     const int np = RGT > 0 && !F32 ? 32 * nw : nw;                // sums an iteration leaves
     sum_t *wsum = reinterpret_cast<sum_t *>(relax_sm);            // [2][np]
     real *P = reinterpret_cast<real *>(wsum + 2 * np);           // [3][RC + 2][W]
+    constexpr bool LEAVE = F32 && RGT > 0;                        // the extra warp forms the FP32 sums
+    constexpr int DR = RGT == 8 ? 1 : 8;                          // slots per group of eight rows
+    float *dev = reinterpret_cast<float *>(P + 3 * plane);       // [2][RC / 8][DR][32 cw]: sums and values left
+    const int dp = gm.RC / 8 * DR * 32 * gm.cw;
     const int r0 = rank * gm.RC, nr = min(gm.RC, Z - r0);        // this block's zone rows (nr <= 0: none)
     real *Pup = nullptr, *Pdn = nullptr;                          // the neighbour blocks' iterates
     sum_t *ptab = nullptr;                                        // block `lane`'s table
@@ -2566,6 +2584,8 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
             }
         }
     }
+    if constexpr (LEAVE)
+        for (int k = threadIdx.x; k < 2 * dp; k += blockDim.x) dev[k] = 0.0f;   // rows past the zone stay zero
     cp_async_wait_all();
     if (C > 1) cl.sync(); else __syncthreads();
     int bi = 0, it = 1, last = 0;                                 // bi: buffer of the iterate read
@@ -2598,7 +2618,27 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
         if (adder) {
             if (it > 1) {
                 sum_t t;
-                if constexpr (F32) t = relax_warp_total(lane < np ? wsum[((it - 1) & 1) * np + lane] : 0ull);
+                if constexpr (LEAVE) {
+                    // lane sums of whole 2^24 units and rests, one warp reduction at the end
+                    const float *d = dev + ((it - 1) & 1) * dp + lane;
+                    unsigned hi = 0, lo = 0;
+                    for (int gr = 0; gr < gm.RC / 8; gr++, d += DR * 32 * gm.cw) {
+#pragma unroll 4
+                        for (int k = 0; k < gm.cw; k++) {
+                            float f = d[k * 32];
+                            if constexpr (RGT < 8) {
+#pragma unroll
+                                for (int r = RR; r < 8; r++) f += d[(r * gm.cw + k) * 32];
+                            }
+                            unsigned h, l;
+                            relax_units_of(f, un, h, l);
+                            lo += l;
+                            hi = min(hi + h + (lo >> 24), RELAX_CAP);
+                            lo &= 0xffffffu;
+                        }
+                    }
+                    t = relax_warp_total(hi, lo);
+                } else if constexpr (F32) t = relax_warp_total(lane < np ? wsum[((it - 1) & 1) * np + lane] : 0ull);
                 else t = warp_sum_fixed(wsum + ((it - 1) & 1) * np, np);
                 if (ptab) ptab[((it - 1) & 1) * 16 + rank] = t;
             }
@@ -2666,7 +2706,11 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
                         Pn[(r + 1) * W + c] = pn;
                         if (r == 0 && Pup) Pup[bo * plane + (gm.RC + 1) * W + c] = pn;
                         if (r == gm.RC - 1 && Pdn) Pdn[bo * plane + c] = pn;
-                        if constexpr (F32) facc += fabsf(pn - u1c);
+                        if constexpr (LEAVE && RGT < 8) {
+                            const float e = fabsf(pn - u1c);
+                            if ((ra & 7) == 0) facc += e;
+                            else dev[(it & 1) * dp + (r * gm.cw + col) * 32 + lane] = e;
+                        } else if constexpr (F32) facc += fabsf(pn - u1c);
                         else acc += fabs((double)pn - (double)u1c) * a.scale;
                     }
                     u0l = u1l; u0c = u1c; u0r = u1r;
@@ -2686,9 +2730,12 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
                         }
                     }
                 }
-                if constexpr (F32) units += relax_warp_total(facc, un);
+                if constexpr (LEAVE) {
+                    if ((ra & 7) == 0) dev[(it & 1) * dp + ((ra >> 3) * DR * gm.cw + col) * 32 + lane] = facc;
+                } else if constexpr (F32) units += relax_warp_total(facc, un);
             }
-            if constexpr (F32) {
+            if constexpr (LEAVE) {
+            } else if constexpr (F32) {
                 if (lane == 0) wsum[(it & 1) * np + warp] = units;
             } else if constexpr (RGT > 0) {
                 wsum[(it & 1) * np + threadIdx.x] = acc;
@@ -2884,7 +2931,8 @@ struct Fused {
     typedef typename Cplx<real>::type cx;
     pfag_ctx *c;
     FusedRes *r;
-    explicit Fused(pfag_ctx *ctx) : c(ctx), r(F(ctx)) {}
+    cudaStream_t bs;        // the spectral passes' stream: the context's, or its own (split)
+    explicit Fused(pfag_ctx *ctx) : c(ctx), r(F(ctx)), bs(ctx->stream) {}
     real *R(void *p) { return (real *)p; }
 
     int configure() {
@@ -2949,8 +2997,11 @@ struct Fused {
             const long strips = (long)c->Ntot * r->tpc;
             r->coop_r = (int)std::max(1L, std::min((long)r->coop_r, strips));
             const long tiles = (long)((c->N + LUM_LRI - 1) / LUM_LRI) * ((c->N + FT - 1) / FT);
-            PFAG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kf_lum_loops<real>, FT, 0));
-            r->coop_l = (int)std::max(1L, std::min((long)nsm * std::min(std::max(per, 1), 8), tiles));
+            // at most one block per SM for the lumen / ECM loops: a cooperative launch
+            // waits until all its blocks fit beside the other stream's kernels, and
+            // it nearly always has nothing left to do (twelve-member sweep: 880 us a
+            // step with every co-resident block, 854 so)
+            r->coop_l = (int)std::max(1L, std::min((long)nsm, tiles));
         }
         PFAG_TRY(choose_clusters(nsm));
         r->ntl = ((c->N + LRB - 1) / LRB) * ((c->N + FT - 1) / FT);
@@ -2973,39 +3024,37 @@ struct Fused {
     }
 
     // Geometry of kf_relax_cells for zones of Z x Z sites: rows split over at
-    // most C blocks, 31 columns a warp, at most g row groups, one more warp for
-    // the sums.  FP32: whole groups of eight rows per block and per warp.
-    bool relax_geom(int C, int g, RelaxGeom &gm, size_t &smem) const {
+    // most C blocks (FP32: whole groups of eight), 31 columns x RG rows a warp,
+    // one more warp for the sums.  False when the block would be too large.
+    // FP32 forms of fewer than 8 rows a warp: blocks of one group only.
+    bool relax_geom(int C, int RG, int RGT, RelaxGeom &gm, size_t &smem) const {
         constexpr bool F32 = sizeof(real) == 4;
         constexpr int U = F32 ? 8 : 1;
         const int Z = 2 * c->zone;
         gm.RC = U * ((Z + C * U - 1) / (C * U));
         gm.C = (Z + gm.RC - 1) / gm.RC;
         gm.cw = (Z + RELAX_COLS - 1) / RELAX_COLS;
-        // the normals in registers when a warp has few enough rows
-        int maxw = RelaxMax<real, 8>::THREADS / 32 - 1;
-        for (int pass = 0; pass < 2; pass++) {
-            gm.g = std::min({g, maxw / gm.cw, gm.RC / U});
-            if (gm.g >= 1) {
-                gm.RG = U * ((gm.RC / U + gm.g - 1) / gm.g);
-                gm.g = (gm.RC + gm.RG - 1) / gm.RG;
-                gm.RGT = F32 ? (gm.RG == 8 ? 8 : 0) : (gm.RG <= 4 ? gm.RG : 0);
-                if (gm.RGT > 0 || pass == 1) break;
-            }
-            maxw = RelaxMax<real, 0>::THREADS / 32 - 1;
-        }
-        if (gm.g < 1) return false;
-        if (gm.RGT == 8 && 32 * (gm.cw * gm.g + 1) > RelaxMax<real, 8>::THREADS) gm.RGT = 0;
+        gm.RG = RG;
+        gm.RGT = RGT;
+        gm.g = (gm.RC + RG - 1) / RG;
         const int nw = gm.cw * gm.g;
-        smem = (size_t)2 * (gm.RGT && !F32 ? 32 * nw : nw) * sizeof(double) +
-               (size_t)3 * (gm.RC + 2) * (Z + 2) * sizeof(real);
+        if (F32 && RGT > 0 && RGT < 8 && gm.RC > 8) return false;
+        if (32 * (nw + 1) > relax_threads(RGT)) return false;
+        smem = (size_t)2 * (RGT && !F32 ? 32 * nw : nw) * sizeof(double) +
+               (size_t)3 * (gm.RC + 2) * (Z + 2) * sizeof(real) +
+               (F32 && RGT > 0 ? (size_t)2 * gm.RC / 8 * (RGT == 8 ? 1 : 8) * 32 * gm.cw * sizeof(float) : 0);
         return smem <= 226 * 1024;
+    }
+    static int relax_threads(int RGT) {
+        return RGT == 0 ? RelaxMax<real, 0>::THREADS : RGT == 4 ? RelaxMax<real, 4>::THREADS
+             : RGT == 2 ? RelaxMax<real, 2>::THREADS : RelaxMax<real, 8>::THREADS;
     }
     typedef void (*relax_fn)(real *, const real *, const real *, const int *, const int *, ReshArgs, RelaxGeom,
                              RelaxUnits, const int4 *, long long *);
     static relax_fn relax_kernel(int RGT) {
         if constexpr (sizeof(real) == 4) {
-            return RGT == 8 ? kf_relax_cells<real, 8> : kf_relax_cells<real, 0>;
+            return RGT == 8 ? kf_relax_cells<real, 8> : RGT == 4 ? kf_relax_cells<real, 4>
+                 : RGT == 2 ? kf_relax_cells<real, 2> : kf_relax_cells<real, 0>;
         } else {
             switch (RGT) {
             case 1: return kf_relax_cells<real, 1>;
@@ -3042,7 +3091,7 @@ struct Fused {
         static std::map<std::array<long, 5>, int> known;
         int dev = 0;
         PFAG_CUDA_CHECK(cudaGetDevice(&dev));
-        const std::array<long, 5> key = {dev, (long)fn, gm.C, gm.cw * gm.g, (long)smem};
+        const std::array<long, 5> key = {(long)dev, (long)fn, (long)gm.C, (long)(gm.cw * gm.g), (long)smem};
         std::lock_guard<std::mutex> lock(mu);
         const auto hit = known.find(key);
         if (hit != known.end()) {
@@ -3067,18 +3116,29 @@ struct Fused {
     // of 258 x 258 at 2 to 3 iterations took 437 us a step against 356 with
     // iteration 1 at full occupancy and the persistent kernel, which organoids
     // with that many cells keep.  Within a size the most row groups that stay
-    // resident.
+    // resident.  The form that reads the normals again, where registers could
+    // hold them in a larger block, only up to 2.5 blocks per SM: 64 cells of 130
+    // x 130 at one iteration took 78 us so, 25 with iteration 1 at full occupancy
+    // and the persistent kernel; the sweep's members of 29 to 37 such cells gain
+    // (twelve members 3.38 -> 2.96 ms for four steps).
     int choose_clusters(int nsm) {
         r->clusters = false;
         if (sizeof(real) == 4 && !relax_units(r->ru)) return PFAG_OK;
+        constexpr bool F32 = sizeof(real) == 4;
         for (int C = 16; C >= 8; C /= 2) {
-            int tried = 0;
-            for (int g = 32; g >= 1; g--) {
+            bool regs = false;     // some form keeps the normals in registers
+            for (int k = 1; k <= 128; k++) {
+                // FP32: 2, 4, 8 rows a warp in registers, then 8, 16, ... without;
+                // FP64: 1 .. 4, then 5, 6, ...
+                const int RG = F32 ? (k <= 3 ? 1 << k : 8 * (k - 3)) : k;
+                const int RGT = F32 ? (k <= 3 ? RG : 0) : (k <= 4 ? k : 0);
                 RelaxGeom gm{};
                 size_t smem = 0;
                 bool fits = false;
-                if (!relax_geom(C, g, gm, smem) || gm.g == tried) continue;   // gm.g <= g: the next form
-                tried = gm.g;
+                if (!relax_geom(C, RG, RGT, gm, smem)) continue;
+                if (RGT == 0 && regs && 2L * c->Ntot * gm.C > 5L * nsm) break;
+                if (RGT == 0 && gm.g == 1 && RG > gm.RC) break;
+                regs = true;
                 PFAG_TRY(relax_resident(gm, smem, nsm, &fits));
                 if (fits) {
                     r->rg = gm;
@@ -3171,6 +3231,12 @@ struct Fused {
         PFAG_CUDA_CHECK(cudaEventCreateWithFlags(&r->ev_boxA, cudaEventDisableTiming));
         PFAG_CUDA_CHECK(cudaEventCreateWithFlags(&r->ev_area, cudaEventDisableTiming));
         PFAG_CUDA_CHECK(cudaEventCreateWithFlags(&r->ev_lum, cudaEventDisableTiming));
+        r->split = (long)c->Ntot * c->M * c->M <= SPLIT_SITES;
+        if (r->split) {
+            PFAG_CUDA_CHECK(cudaStreamCreateWithFlags(&r->spec, cudaStreamNonBlocking));
+            PFAG_CUDA_CHECK(cudaEventCreateWithFlags(&r->ev_upd, cudaEventDisableTiming));
+            PFAG_CUDA_CHECK(cudaEventCreateWithFlags(&r->ev_spec, cudaEventDisableTiming));
+        }
         PFAG_CUDA_CHECK(cudaMalloc(&r->cK, sizeof(int) * (3 * c->Ntot + 8)));
         r->cdone = r->cK + c->Ntot;
         r->ccnt = r->cK + 2 * c->Ntot;
@@ -3238,6 +3304,19 @@ struct Fused {
                                                      R(r->Jc), R(r->G));
         }
         PFAG_LAUNCHED(c);
+        return PFAG_OK;
+    }
+
+    // after the pass that reads phi, rho, lum and ECM: what waits for it (the
+    // lumen / ECM relaxation, the cells' loops), and the phi update where it
+    // shares the spectral passes' stream
+    int after_pass_a() {
+        if (r->fork) PFAG_CUDA_CHECK(cudaEventRecord(r->ev_boxA, bs));
+        return bs == c->stream ? launch_update() : PFAG_OK;
+    }
+    // before the pass that writes the new rho in place: the phi update reads the old one
+    int before_new_rho() {
+        if (bs != c->stream) PFAG_CUDA_CHECK(cudaStreamWaitEvent(bs, r->ev_upd, 0));
         return PFAG_OK;
     }
 
@@ -3316,6 +3395,13 @@ struct Fused {
         // 4-5. spectral solve with the phi update after its pass A; the last
         //    column pass writes the new rho over each box in place
         //    (rho <- rhon of run_with_active_gels.cpp:175-178 on the box)
+        const bool split = fork && r->split;
+        if (split) {
+            bs = r->spec;
+            PFAG_CUDA_CHECK(cudaStreamWaitEvent(bs, r->ev_psi, 0));
+            PFAG_TRY(launch_update());
+            PFAG_CUDA_CHECK(cudaEventRecord(r->ev_upd, s));
+        }
         const BoxArgs ba = box_args(c);
         const int Rr = r->rows_blk, G = r->grp_cols;
         cx *Y1 = (cx *)r->Y1, *Y2 = (cx *)r->Y2;
@@ -3326,23 +3412,23 @@ struct Fused {
         else if (M == 32) { PFAG_TRY(box_reg<32>(ba)); }
         else {
         pfag_prof_begin(c, "kf_boxA");
-        kf_boxA<real><<<dim3(M / Rr, Nt), FT, r->smemA, s>>>(R(c->phi), R(c->rho), R(c->lum), R(c->ecm), c->d_xc,
+        kf_boxA<real><<<dim3(M / Rr, Nt), FT, r->smemA, bs>>>(R(c->phi), R(c->rho), R(c->lum), R(c->ecm), c->d_xc,
                                                              c->d_yc, ba, Rr, Y1, Y2, R(r->Rb), r->clsT);
         PFAG_LAUNCHED(c);
-        if (r->fork) PFAG_CUDA_CHECK(cudaEventRecord(r->ev_boxA, s));
-        PFAG_TRY(launch_update());
+        PFAG_TRY(after_pass_a());
         const int ngrp = (M / 2 + 1 + G - 1) / G;
         pfag_prof_begin(c, "kf_boxB");
-        kf_boxB<real><<<dim3(ngrp, Nt), FT, r->smemB, s>>>(Y1, Y2, r->clsT, ba, G); PFAG_LAUNCHED(c);
+        kf_boxB<real><<<dim3(ngrp, Nt), FT, r->smemB, bs>>>(Y1, Y2, r->clsT, ba, G); PFAG_LAUNCHED(c);
         pfag_prof_begin(c, "kf_boxC");
-        kf_boxC<real><<<dim3(M / Rr, Nt), FT, r->smemC, s>>>(Y1, Y2, R(c->rho), c->d_xc, c->d_yc, ba, Rr,
+        kf_boxC<real><<<dim3(M / Rr, Nt), FT, r->smemC, bs>>>(Y1, Y2, R(c->rho), c->d_xc, c->d_yc, ba, Rr,
                                                              c->debug ? R(c->d_vx) : nullptr,
                                                              c->debug ? R(c->d_vy) : nullptr);
         PFAG_LAUNCHED(c);
         pfag_prof_begin(c, "kf_boxD");
-        kf_boxD<real><<<dim3(ngrp, Nt), FT, r->smemD, s>>>(Y1, Y2, ba, G); PFAG_LAUNCHED(c);
+        kf_boxD<real><<<dim3(ngrp, Nt), FT, r->smemD, bs>>>(Y1, Y2, ba, G); PFAG_LAUNCHED(c);
+        PFAG_TRY(before_new_rho());
         pfag_prof_begin(c, "kf_boxE");
-        kf_boxE<real><<<dim3(M / Rr, Nt), FT, r->smemE, s>>>(Y1, R(c->rho), R(r->Rb), R(c->rho), c->d_xc, c->d_yc,
+        kf_boxE<real><<<dim3(M / Rr, Nt), FT, r->smemE, bs>>>(Y1, R(c->rho), R(r->Rb), R(c->rho), c->d_xc, c->d_yc,
                                                              ba, Rr);
         PFAG_LAUNCHED(c);
         }
@@ -3389,6 +3475,10 @@ struct Fused {
         // 7. reshaping of the cells: a cluster per cell; where not every cell's
         //    cluster is resident, iteration 1 at full occupancy and the persistent
         //    kernel, after the join
+        if (split) {
+            PFAG_CUDA_CHECK(cudaEventRecord(r->ev_spec, bs));
+            PFAG_CUDA_CHECK(cudaStreamWaitEvent(s, r->ev_boxA, 0));    // pass A reads the phi written next
+        }
         {
             ReshArgs ra{};
             ra.N = N; ra.z = z; ra.Ntot = Nt; ra.tpc = r->tpc;
@@ -3426,6 +3516,7 @@ struct Fused {
                 PFAG_LAUNCHED(c);
             }
         }
+        if (split) PFAG_CUDA_CHECK(cudaStreamWaitEvent(s, r->ev_spec, 0));
         // 8. periodic ghost ring of rho (boundary_conditions_cells(rhon),
         //    rho_functions.cpp:469).  Its sources, rows and columns 1 and N-2,
         //    lie outside every box (boxes span [xc-z+1, xc+z-2] with
@@ -3441,6 +3532,13 @@ struct Fused {
 
     // zone rows per reshaping strip
     static constexpr int RESH_RB = 8;
+    // largest organoid (box sites of all cells) whose spectral passes run beside
+    // the phi update and the cells' loops, which leave most of the GPU idle there
+    // (us a step, one after the other and side by side: 3 x 32^2 94 and 81, 7 x
+    // 128^2 120 and 89, 19 x 114^2 100 and 85, 6 x 398^2 266 and 232, 64 x 128^2
+    // 259 and 245); at 64 x 256^2 every pass fills the GPU and they only contend
+    // (349 and 363)
+    static constexpr long SPLIT_SITES = 2L << 20;
     // lumen/ECM relaxation iterations run as regular kernels before the persistent one
     static constexpr int LUM_REGULAR = 2;
 
@@ -3464,7 +3562,7 @@ struct Fused {
     template <int L>
     int box_blue(const BoxArgs &ba) {
         typedef BlueGeom<real, L> BGm;
-        cudaStream_t s = c->stream;
+        cudaStream_t s = bs;
         const int M = c->M, Nt = c->Ntot, N = c->N, z = c->zone, H = M / 2 + 1;
         cx *Y1 = (cx *)r->Y1, *Y2 = (cx *)r->Y2, *Hs = (cx *)r->Gsp;
         const BlueTabs<cx> tb = blue_tabs();
@@ -3486,8 +3584,7 @@ struct Fused {
         kg_stress<real><<<g, 256, 0, s>>>(R(c->phi), R(c->rho), R(c->lum), R(c->ecm), c->d_xc, c->d_yc, ba, Y1, Y2,
                                           R(r->Rb), r->clsT);
         PFAG_LAUNCHED(c);
-        if (r->fork) PFAG_CUDA_CHECK(cudaEventRecord(r->ev_boxA, s));
-        PFAG_TRY(launch_update());
+        PFAG_TRY(after_pass_a());
         {
             const long tasks = (long)Nt * (M + M / 2);
             pfag_prof_begin(c, "kbl_rowsA");
@@ -3529,6 +3626,7 @@ struct Fused {
             kbl_colsE<real, L><<<(unsigned)tasks, BGm::THREADS, sm_colsE, s>>>(X, M, Nt, tb);
             PFAG_LAUNCHED(c);
         }
+        PFAG_TRY(before_new_rho());
         pfag_prof_begin(c, "kbl_rho");
         kbl_rho<real><<<g, 256, 0, s>>>(X, R(c->rho), c->d_xc, c->d_yc, N, z, M, Nt);
         PFAG_LAUNCHED(c);
@@ -3552,7 +3650,7 @@ struct Fused {
     template <int MM>
     int box_reg(const BoxArgs &ba) {
         typedef BoxGeom<MM> BG;
-        cudaStream_t s = c->stream;
+        cudaStream_t s = bs;
         const int Nt = c->Ntot;
         const size_t cs = sizeof(cx);
         const size_t smA = (MM + (size_t)BG::ROWS * MM) * cs + (size_t)BG::ROWS * MM * sizeof(real) +
@@ -3574,8 +3672,7 @@ struct Fused {
         kr_boxA<real, MM><<<grow, BG::THREADS, smA, s>>>(R(c->phi), R(c->rho), R(c->lum), R(c->ecm), c->d_xc, c->d_yc,
                                                           ba, Y1, Y2, R(r->Rb), r->clsT);
         PFAG_LAUNCHED(c);
-        if (r->fork) PFAG_CUDA_CHECK(cudaEventRecord(r->ev_boxA, s));
-        PFAG_TRY(launch_update());
+        PFAG_TRY(after_pass_a());
         pfag_prof_begin(c, "kr_boxB");
         kr_boxB<real, MM, GB, 256><<<dim3((MM / 2 + 1 + GB - 1) / GB, Nt), 256, smB, s>>>(Y1, Y2, r->clsT, ba);
         PFAG_LAUNCHED(c);
@@ -3585,6 +3682,7 @@ struct Fused {
                                                            c->debug ? R(c->d_vx) : nullptr,
                                                            c->debug ? R(c->d_vy) : nullptr);
         PFAG_LAUNCHED(c);
+        PFAG_TRY(before_new_rho());
         pfag_prof_begin(c, "kr_boxD2");
         kr_boxD2<real, MM><<<dim3(MM / BD::COLS, Nt), 256, smD2, s>>>(X, R(c->rho), R(r->Rb), c->d_xc, c->d_yc, ba);
         PFAG_LAUNCHED(c);
