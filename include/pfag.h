@@ -318,6 +318,13 @@ int pfag_conv3x3(const void *x, const void *w, const float *bias, void *y, void 
  * sum of dz[q][co] (accumulates: zero dw, db first). */
 int pfag_conv3x3_wgrad(const void *x, const void *dz, float *dw, float *db, int B, int H, int W, int cin,
                        int cout, unsigned *err, void *stream);
+/* dx = the input gradient of that layer from dz (BF16 [B][H+2][W+2][cout]),
+ * rounded to BF16, and with gelu_on times GELU'(pre), pre the pre-activation
+ * of the layer below (BF16 [B][H+2][W+2][cin]), rounded again: what
+ * pfag_conv_flip, pfag_conv3x3 of dz and pfag_conv_act_bwd give, in one kernel.
+ * The halo rows of dx are not written. */
+int pfag_conv3x3_dgrad(const void *dz, const void *w, const void *pre, void *dx, int B, int H, int W, int cin,
+                       int cout, int gelu_on, unsigned *err, void *stream);
 /* dz = dy * GELU'(pre) (gelu_on) or dy, zero on the halo. */
 int pfag_conv_act_bwd(const void *dy, const void *pre, void *dz, int B, int H, int W, int c, int gelu_on,
                       void *stream);
@@ -328,6 +335,10 @@ int pfag_conv_flip(const void *w, void *wt, int cin, int cout, void *stream);
  * (optional) multiplies each update. */
 int pfag_adam(float *p, const float *g, float *m, float *v, void *pb, const float *mask, int n, float lr,
               float b1, float b2, float eps, int t, void *stream);
+/* pfag_adam without masks on 1 to 16 tensors in one launch (host arrays of
+ * device pointers and lengths; pb[k] may be NULL). */
+int pfag_adam_list(int count, float *const *p, const float *const *g, float *const *m, float *const *v,
+                   void *const *pb, const int *n, float lr, float b1, float b2, float eps, int t, void *stream);
 /* Squared error of the first nout channels of out (C = 16 channels) against
  * target [B][H][W][nout] (FP32): *loss += the sum, dout = 2 scale (out -
  * target) on those channels and sites, zero elsewhere. */

@@ -66,6 +66,7 @@ EXPORTS = [
     "pfag_seed_organoid", "pfag_set_launch_shape", "pfag_batch_create", "pfag_batch_step", "pfag_batch_step_async", "pfag_batch_sync",
     "pfag_batch_stream", "pfag_batch_launch_count", "pfag_batch_destroy",
     "pfag_upload_device", "pfag_conv3x3", "pfag_conv3x3_wgrad", "pfag_conv_act_bwd", "pfag_conv_flip", "pfag_adam",
+    "pfag_conv3x3_dgrad", "pfag_adam_list",
     "pfag_conv_mse", "pfag_corrector_gather", "pfag_corrector_apply",
     "pfag_shard_enable", "pfag_step_head", "pfag_step_tail", "pfag_sum_planes", "pfag_device_field",
     "pfag_set_lumen_tiles",
@@ -125,6 +126,8 @@ def lib() -> ctypes.CDLL:
         L.pfag_upload_device.argtypes = [vp, vp, vp, vp, vp]
         L.pfag_conv3x3.argtypes = [vp, vp, vp, vp, vp, i, i, i, i, i, i, vp, vp]
         L.pfag_conv3x3_wgrad.argtypes = [vp, vp, vp, vp, i, i, i, i, i, vp, vp]
+        L.pfag_conv3x3_dgrad.argtypes = [vp, vp, vp, vp, i, i, i, i, i, i, vp, vp]
+        L.pfag_adam_list.argtypes = [i, vp, vp, vp, vp, vp, vp, f, f, f, f, i, vp]
         L.pfag_conv_act_bwd.argtypes = [vp, vp, vp, i, i, i, i, i, vp]
         L.pfag_conv_flip.argtypes = [vp, vp, i, i, vp]
         L.pfag_adam.argtypes = [vp, vp, vp, vp, vp, vp, i, f, f, f, f, i, vp]

@@ -119,33 +119,34 @@ class ConvNet:
         dout = self._buf("dout", out.shape)
         capi.check(L.pfag_conv_mse(_p(out), _p(target), _p(dout), _p(loss), B, H, W, 16, REAL_OUT,
                                    1.0 / (B * H * W * REAL_OUT), _stream()))
+        # one zeroed buffer for every layer's weight and bias gradients
+        flat = torch.zeros(sum(w.numel() + b.numel() for w, b in zip(self.W, self.b)), device="cuda")
+        parts = iter(flat.split([t.numel() for pair in zip(self.W, self.b) for t in pair]))
+        gW, gb = zip(*[(next(parts), next(parts)) for _ in LAYERS])
         dz = dout
-        grads = []
         for k in range(len(LAYERS) - 1, -1, -1):
             cin, cout, act = LAYERS[k]
-            dw = torch.zeros_like(self.W[k])
-            db = torch.zeros_like(self.b[k])
-            capi.check(L.pfag_conv3x3_wgrad(_p(self.acts[k]), _p(dz), _p(dw), _p(db), B, H, W, cin, cout,
+            capi.check(L.pfag_conv3x3_wgrad(_p(self.acts[k]), _p(dz), _p(gW[k]), _p(gb[k]), B, H, W, cin, cout,
                                             _p(self.err), _stream()))
-            grads.append((k, dw, db))
             if k == 0:
                 break
-            wt = self._buf(("wt", k), (cin, 9, cout))
-            capi.check(L.pfag_conv_flip(_p(self.Wb[k]), _p(wt), cin, cout, _stream()))
-            da = self._buf(("da", k), (B, H + 2, W + 2, cin))
-            zero_b = self._buf(("zb", cin), (cin,), torch.float32)
-            capi.check(L.pfag_conv3x3(_p(dz), _p(wt), _p(zero_b), _p(da), None, B, H, W, cout, cin, 0, _p(self.err),
-                                      _stream()))
+            # the gradient below this layer, times the GELU's derivative there
             pcin, pcout, pact = LAYERS[k - 1]
-            dz = self._buf(("dz", k - 1), (B, H + 2, W + 2, pcout))
-            capi.check(L.pfag_conv_act_bwd(_p(da), _p(self.pres[k - 1]), _p(dz), B, H, W, pcout, 1 if pact else 0,
-                                           _stream()))
+            below = self._buf(("dz", k - 1), (B, H + 2, W + 2, pcout))
+            pre = self.pres[k - 1]
+            capi.check(L.pfag_conv3x3_dgrad(_p(dz), _p(self.Wb[k]), _p(pre) if pact else None, _p(below), B, H, W, cin,
+                                            cout, 1 if pact else 0, _p(self.err), _stream()))
+            dz = below
         self.t += 1
-        for k, dw, db in grads:
-            capi.check(L.pfag_adam(_p(self.W[k]), _p(dw), _p(self.mW[k]), _p(self.vW[k]), _p(self.Wb[k]), None,
-                                   self.W[k].numel(), lr, 0.9, 0.999, 1e-8, self.t, _stream()))
-            capi.check(L.pfag_adam(_p(self.b[k]), _p(db), _p(self.mb[k]), _p(self.vb[k]), None, None,
-                                   self.b[k].numel(), lr, 0.9, 0.999, 1e-8, self.t, _stream()))
+        n = 2 * len(LAYERS)
+
+        def ptrs(*groups):
+            return (ctypes.c_void_p * n)(*[t.data_ptr() if t is not None else None for g in zip(*groups) for t in g])
+
+        sizes = (ctypes.c_int * n)(*[t.numel() for pair in zip(self.W, self.b) for t in pair])
+        capi.check(L.pfag_adam_list(n, ptrs(self.W, self.b), ptrs(gW, gb), ptrs(self.mW, self.mb),
+                                    ptrs(self.vW, self.vb), ptrs(self.Wb, [None] * len(LAYERS)), sizes, lr, 0.9, 0.999,
+                                    1e-8, self.t, _stream()))
         return loss / (B * H * W * REAL_OUT)
 
     def check_err(self):
