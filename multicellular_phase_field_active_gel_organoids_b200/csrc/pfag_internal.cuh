@@ -87,6 +87,8 @@ struct pfag_ctx {
     void *maps[6];  // deg, gen, a_tan, a_ort, visc, b
     void *pixx, *pixy, *piyy;
     void *fftbuf;   // 11 * Ntot * M*M complex
+    void *cell_t, *lum_t;   // the plain loops' second iterate: [Ntot][2z][2z], [N][N]
+    double *part_z;         // their blocks' sums
     cufftHandle plan;
     bool plan_ok;
     // small device arrays

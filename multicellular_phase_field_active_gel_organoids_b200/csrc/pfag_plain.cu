@@ -3,6 +3,7 @@
 // cells).  This is the FP64 comparison path and what the drop-in layer calls
 // function by function.  Each kernel cites the reference loop it computes.
 #include "pfag_internal.cuh"
+#include <algorithm>
 #include <cmath>
 
 namespace {
@@ -257,7 +258,7 @@ __global__ void k_serial_absdiff(const real *__restrict__ a, const real *__restr
 }
 
 template <typename real>
-__global__ void k_serial_cell_rdev(const real *__restrict__ pn, const real *__restrict__ p,
+__global__ void k_serial_cell_rdev(const real *__restrict__ pn, const real *__restrict__ p, bool compact,
                                    const int *__restrict__ xc, const int *__restrict__ yc, int N, int z, int ncells,
                                    double dx, double ncur, const int *__restrict__ active,
                                    double *__restrict__ out) {
@@ -268,7 +269,8 @@ __global__ void k_serial_cell_rdev(const real *__restrict__ pn, const real *__re
         for (int i = xc[n] - z; i < xc[n] + z; i++)
             for (int j = yc[n] - z; j < yc[n] + z; j++) {
                 const size_t o = cidx(n, i, j, N);
-                acc += fabs((double)pn[o] - (double)p[o]) * dx * dx / ncur;
+                const size_t t = compact ? cidx(n, i - xc[n] + z, j - yc[n] + z, 2 * z) : o;   // [Ntot][2z][2z]
+                acc += fabs((double)pn[t] - (double)p[o]) * dx * dx / ncur;
             }
     out[n] = acc;
 }
@@ -484,28 +486,60 @@ __global__ void k_lum_normals(const real *__restrict__ lumn, const real *__restr
     jy[c] = (g != (real)0.0) ? inv2dx * (lumn[c + 1] - lumn[c - 1]) / g : (real)0.0;
 }
 
-// one relaxation update of the lumen/ECM field (interior), :802-838
+// One iteration of the lumen/ECM loop (:774-849): f <- P, Q = P + its
+// relaxation update (interior; :802-838), the Dirichlet values on the boundary
+// (useful_functions.cpp:422-437), and the block's sum of |Q - P| dx^2.  Does
+// nothing once the loop has stopped (*active == 0).
 template <typename real>
-__global__ void k_lum_relax(const real *__restrict__ p, real *__restrict__ pn, const real *__restrict__ jx,
-                            const real *__restrict__ jy, int N, real A, real B) {
-    const int i = 1 + blockIdx.y * TBY + threadIdx.y, j = 1 + blockIdx.x * TBX + threadIdx.x;
-    if (i > N - 2 || j > N - 2) return;
-    const size_t c = (size_t)i * N + j;
-    real q[3][3];
-    for (int a = 0; a < 3; a++)
-        for (int b = 0; b < 3; b++) q[a][b] = p[c + (size_t)(a - 1) * N + (b - 1)];
-    pn[c] = resh_update<real>(A, B, q, jx[c], jx[c + N], jx[c - N], jx[c + 1], jx[c - 1], jy[c], jy[c + N],
-                              jy[c - N], jy[c + 1], jy[c - 1], pn[c]);
+__global__ void k_lum_iter(const real *__restrict__ p, real *__restrict__ q, real *__restrict__ f,
+                           const real *__restrict__ jx, const real *__restrict__ jy, int N, real A, real B, real side,
+                           double scale, const int *__restrict__ active, double *__restrict__ part) {
+    if (!*active) return;
+    const int i = blockIdx.y * TBY + (threadIdx.x >> 5), j = blockIdx.x * TBX + (threadIdx.x & 31);
+    double acc = 0.0;
+    if (i < N && j < N) {
+        const size_t c = (size_t)i * N + j;
+        const real old = p[c];
+        const bool ei = i == 0 || i == N - 1, ej = j == 0 || j == N - 1;
+        real v;
+        if (ei || ej) {
+            v = ei && ej ? (real)0.0 : side;
+        } else {
+            real w[3][3];
+            for (int a = 0; a < 3; a++)
+                for (int b = 0; b < 3; b++) w[a][b] = p[c + (size_t)(a - 1) * N + (b - 1)];
+            v = resh_update<real>(A, B, w, jx[c], jx[c + N], jx[c - N], jx[c + 1], jx[c - 1], jy[c], jy[c + N],
+                                  jy[c - N], jy[c + 1], jy[c - 1], old);
+        }
+        q[c] = v;
+        f[c] = old;
+        acc = fabs((double)v - (double)old) * scale;
+    }
+    const double r = block_sum(acc);
+    if (threadIdx.x == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = r;
 }
 
+// The loop's end test after it (:851-868): rdev from the blocks' sums in a fixed
+// order.  st: [0] active, [1] ri, [2] iterations, [3] passed rimax.
+__global__ void k_lum_check(const double *__restrict__ part, int npart, double thr, int rimax, int *__restrict__ st) {
+    if (!st[0]) return;
+    double a = 0.0;
+    for (int k = threadIdx.x; k < npart; k += blockDim.x) a += part[k];
+    a = block_sum(a);
+    if (threadIdx.x == 0) {
+        st[2]++;
+        bool stop = !(a > thr);
+        if (st[1] > rimax) { st[3] = 1; stop = true; }
+        else st[1]++;
+        if (stop) st[0] = 0;
+    }
+}
+// the last iterate back into fn after an odd iteration count
 template <typename real>
-__global__ void k_absdiff_sum(const real *__restrict__ a, const real *__restrict__ b, size_t ng, double scale,
-                              double *__restrict__ part) {
-    double acc = 0.0;
-    for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < ng; k += (size_t)gridDim.x * blockDim.x)
-        acc += fabs((double)a[k] - (double)b[k]) * scale;
-    double r = block_sum(acc);
-    if (threadIdx.x == 0) part[blockIdx.x] = r;
+__global__ void k_lum_last(real *__restrict__ fn, const real *__restrict__ q, size_t n, const int *__restrict__ st) {
+    if (!(st[2] & 1)) return;
+    for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
+        fn[k] = q[k];
 }
 
 __global__ void k_sum_partials(const double *__restrict__ part, int nblk, double *__restrict__ out) {
@@ -569,72 +603,75 @@ __global__ void k_update_cells(const real *__restrict__ phi, real *__restrict__ 
 }
 
 // ---- reshaping_cells (cell_phase_functions.cpp:447-580) ---------------------
-// active[n] != 0 while cell n is still iterating.
-template <typename real>
-__global__ void k_zone_copy(real *__restrict__ dst, const real *__restrict__ src, const int *__restrict__ xc,
-                            const int *__restrict__ yc, int N, int z, const int *__restrict__ active) {
+// Iteration k takes iterate k - 1 to iterate k: odd ones from phin into the
+// compact planes T ([Ntot][2z][2z]), even ones back, so that reading and
+// writing need no copy between them; each stores its input into phi (the copy
+// at the top of the reference's loop).  active[n] != 0 while cell n is still
+// iterating; a stopped cell's blocks return at once, so the host can enqueue
+// several iterations between its looks at the flags.
+template <typename real, bool ODD>
+__global__ void k_cell_iter(real *__restrict__ phi, real *__restrict__ phin, real *__restrict__ T,
+                            const real *__restrict__ jx, const real *__restrict__ jy, const int *__restrict__ xc,
+                            const int *__restrict__ yc, int N, int z, real A, real B, double scale,
+                            const int *__restrict__ active, double *__restrict__ part) {
     const int n = blockIdx.z;
     if (!active[n]) return;
-    const int i = xc[n] - z + blockIdx.y * TBY + threadIdx.y;
-    const int j = yc[n] - z + blockIdx.x * TBX + threadIdx.x;
-    if (i >= xc[n] + z || j >= yc[n] + z) return;
-    dst[cidx(n, i, j, N)] = src[cidx(n, i, j, N)];
-}
-
-template <typename real>
-__global__ void k_cell_relax(const real *__restrict__ p, real *__restrict__ pn, const real *__restrict__ jx,
-                             const real *__restrict__ jy, const int *__restrict__ xc, const int *__restrict__ yc,
-                             int N, int z, real A, real B, const int *__restrict__ active) {
-    const int n = blockIdx.z;
-    if (!active[n]) return;
-    const int i = xc[n] - z + blockIdx.y * TBY + threadIdx.y;
-    const int j = yc[n] - z + blockIdx.x * TBX + threadIdx.x;
-    if (i >= xc[n] + z || j >= yc[n] + z) return;
-    const size_t base = (size_t)n * N * N, c = (size_t)i * N + j;
-    const real *q = p + base, *X = jx + base, *Y = jy + base;
-    real w[3][3];
-    for (int a = 0; a < 3; a++)
-        for (int b = 0; b < 3; b++) w[a][b] = q[c + (size_t)(a - 1) * N + (b - 1)];
-    pn[base + c] = resh_update<real>(A, B, w, X[c], X[c + N], X[c - N], X[c + 1], X[c - 1], Y[c], Y[c + N],
-                                     Y[c - N], Y[c + 1], Y[c - 1], pn[base + c]);
-}
-
-// rdev per active cell: sum over the zone of |phin - phi| dx^2 / N_current
-template <typename real>
-__global__ void k_cell_rdev(const real *__restrict__ pn, const real *__restrict__ p, const int *__restrict__ xc,
-                            const int *__restrict__ yc, int N, int z, double scale, const int *__restrict__ active,
-                            double *__restrict__ part) {
-    const int n = blockIdx.y;
+    const int Z = 2 * z, li = blockIdx.y * TBY + (threadIdx.x >> 5), lj = blockIdx.x * TBX + (threadIdx.x & 31);
     double acc = 0.0;
-    if (active[n]) {
-        const int w = 2 * z;
-        const size_t tot = (size_t)w * w;
-        for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < tot; k += (size_t)gridDim.x * blockDim.x) {
-            const int i = xc[n] - z + (int)(k / w), j = yc[n] - z + (int)(k % w);
-            const size_t o = cidx(n, i, j, N);
-            acc += fabs((double)pn[o] - (double)p[o]) * scale;
-        }
+    if (li < Z && lj < Z) {
+        const size_t base = (size_t)n * N * N, c = (size_t)(xc[n] - z + li) * N + (yc[n] - z + lj);
+        const size_t tb = (size_t)n * Z * Z, tc = (size_t)li * Z + lj;
+        const real *X = jx + base, *Y = jy + base;
+        real w[3][3];
+        for (int a = 0; a < 3; a++)
+            for (int b = 0; b < 3; b++) {
+                // the ring around the zone, which no iteration writes, from phi
+                const int ii = li + a - 1, jj = lj + b - 1;
+                const bool ring = ii < 0 || ii >= Z || jj < 0 || jj >= Z;
+                const size_t o = base + c + (size_t)(a - 1) * N + (b - 1);
+                w[a][b] = ring ? phi[o] : ODD ? phin[o] : T[tb + (size_t)ii * Z + jj];
+            }
+        const real old = w[1][1];
+        const real v = resh_update<real>(A, B, w, X[c], X[c + N], X[c - N], X[c + 1], X[c - 1], Y[c], Y[c + N],
+                                         Y[c - N], Y[c + 1], Y[c - 1], old);
+        if (ODD) T[tb + tc] = v;
+        else phin[base + c] = v;
+        phi[base + c] = old;
+        acc = fabs((double)v - (double)old) * scale;
     }
-    double r = block_sum(acc);
-    if (threadIdx.x == 0) part[(size_t)n * gridDim.x + blockIdx.x] = r;
+    const double r = block_sum(acc);
+    if (threadIdx.x == 0) part[((size_t)n * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = r;
+}
+// the last iterate back into phin for the cells with an odd iteration count
+template <typename real>
+__global__ void k_cell_last(real *__restrict__ phin, const real *__restrict__ T, const int *__restrict__ xc,
+                            const int *__restrict__ yc, int N, int z, const int *__restrict__ iters) {
+    const int n = blockIdx.z, Z = 2 * z;
+    if (!(iters[n] & 1)) return;
+    const int li = blockIdx.y * TBY + (threadIdx.x >> 5), lj = blockIdx.x * TBX + (threadIdx.x & 31);
+    if (li < Z && lj < Z)
+        phin[(size_t)n * N * N + (size_t)(xc[n] - z + li) * N + yc[n] - z + lj] =
+            T[(size_t)n * Z * Z + (size_t)li * Z + lj];
 }
 
 // Convergence bookkeeping of the while loop at cell_phase_functions.cpp:475-574:
 // after an iteration, the loop ends when rdev <= thr, or (ri > rimax) breaks.
-__global__ void k_cell_check(const double *__restrict__ part, int nblk, int ncells, double thr, int rimax,
-                             int *__restrict__ active, int *__restrict__ ri, int *__restrict__ nactive,
+// One warp per cell; rdev from the blocks' sums in a fixed order.
+__global__ void k_cell_check(const double *__restrict__ part, int nblk, double thr, int rimax,
+                             int *__restrict__ active, int *__restrict__ ri, int *__restrict__ iters,
                              unsigned *__restrict__ err) {
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= ncells) return;
+    const int n = blockIdx.x;
     if (!active[n]) return;
     double a = 0.0;
-    for (int b = 0; b < nblk; b++) a += part[(size_t)n * nblk + b];
+    for (int b = threadIdx.x; b < nblk; b += 32) a += part[(size_t)n * nblk + b];
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (threadIdx.x != 0) return;
     bool stop = false;
     if (ri[n] > rimax) { atomicOr(err, ERRBIT_RELAX); stop = true; }
     else ri[n]++;
+    iters[n]++;
     if (a <= thr) stop = true;
     if (stop) active[n] = 0;
-    else atomicAdd(nactive, 1);
 }
 
 template <typename real>
@@ -855,19 +892,6 @@ struct Plain {
         k_copy_to_rhon<real><<<bg, tb, 0, s>>>(T, R(c->rhon), c->d_xc, c->d_yc, N, z, M); PFAG_LAUNCHED(c);
         return bc_cells(c->rhon, c->Ntot);
     }
-    int sum_reduce_2d(const void *a, const void *b, double scale, double *out) {
-        if (c->serial_sums) {
-            k_serial_absdiff<real><<<1, 32, 0, c->stream>>>(R((void *)a), R((void *)b), c->N, c->dp.dx, out);
-            PFAG_LAUNCHED(c);
-            return PFAG_OK;
-        }
-        k_absdiff_sum<real><<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(R((void *)a), R((void *)b), c->ng, scale,
-                                                                      c->d_part);
-        PFAG_LAUNCHED(c);
-        k_sum_partials<<<1, 32, 0, c->stream>>>(c->d_part, RED_BLOCKS, out);
-        PFAG_LAUNCHED(c);
-        return PFAG_OK;
-    }
     int lum_ecm_update() {
         const int N = c->N;
         // sum_ecm = sum h(ECM) dx^2 over the full grid (FP64)
@@ -903,25 +927,44 @@ struct Plain {
         PFAG_LAUNCHED(c);
         PFAG_TRY(bc_cells(c->jx, 1));
         PFAG_TRY(bc_cells(c->jy, 1));
-        double rdev = c->dp.rdev0_lum;
-        int ri = 0;
-        const real A = (real)c->dp.A_resh, B = (real)c->dp.B_resh;
-        while (rdev > c->dp.thr_lum) {
-            k_copy<real><<<592, 256, 0, c->stream>>>(R(f), R(fn), c->ng); PFAG_LAUNCHED(c);
-            k_lum_relax<real><<<interior_grid(1), dim3(TBX, TBY), 0, c->stream>>>(R(f), R(fn), R(c->jx), R(c->jy), N,
-                                                                                  A, B);
-            PFAG_LAUNCHED(c);
-            k_dirichlet<real><<<(4 * N + 255) / 256, 256, 0, c->stream>>>(R(fn), N, side, (real)0.0);
-            PFAG_LAUNCHED(c);
-            PFAG_TRY(sum_reduce_2d(fn, f, c->dp.dx * c->dp.dx, c->d_scal + 1));
-            PFAG_CUDA_CHECK(cudaMemcpyAsync(c->h_scal + 1, c->d_scal + 1, sizeof(double), cudaMemcpyDeviceToHost,
-                                            c->stream));
-            PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
-            rdev = c->h_scal[1];
-            if (ri > c->p.rimax) { c->stats.relax_failures++; break; }
-            ri++;
+        // the loop's state on the device: active, ri, iterations, passed rimax; the
+        // host looks at it after LUM_AHEAD iterations enqueued (the ones past
+        // the end do nothing)
+        int *st = c->d_iflags + 8 * c->Ntot, *hst = c->h_iflags + 8 * c->Ntot;
+        hst[0] = c->dp.rdev0_lum > c->dp.thr_lum ? 1 : 0;
+        hst[1] = hst[2] = hst[3] = 0;
+        if (hst[0]) {
+            const real A = (real)c->dp.A_resh, B = (real)c->dp.B_resh;
+            const dim3 g((N + TBX - 1) / TBX, (N + TBY - 1) / TBY);
+            real *T = R(c->lum_t);
+            PFAG_CUDA_CHECK(cudaMemcpyAsync(st, hst, 4 * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+            const int ahead = c->serial_sums ? 1 : LUM_AHEAD;
+            for (int it = 1; hst[0];) {
+                for (int k = 0; k < ahead; k++, it++) {
+                    real *P = (it & 1) ? R(fn) : T, *Q = (it & 1) ? T : R(fn);
+                    k_lum_iter<real><<<g, 256, 0, c->stream>>>(P, Q, R(f), R(c->jx), R(c->jy), N, A, B, side,
+                                                               c->dp.dx * c->dp.dx, st, c->part_z);
+                    PFAG_LAUNCHED(c);
+                    const double *part = c->part_z;
+                    int npart = (int)(g.x * g.y);
+                    if (c->serial_sums) {
+                        k_serial_absdiff<real><<<1, 32, 0, c->stream>>>(Q, R(f), N, c->dp.dx, c->d_scal + 1);
+                        PFAG_LAUNCHED(c);
+                        part = c->d_scal + 1;
+                        npart = 1;
+                    }
+                    k_lum_check<<<1, RED_THREADS, 0, c->stream>>>(part, npart, c->dp.thr_lum, c->p.rimax, st);
+                    PFAG_LAUNCHED(c);
+                }
+                PFAG_CUDA_CHECK(cudaMemcpyAsync(hst, st, 4 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+                PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
+            }
+            if (hst[2] & 1) {
+                k_lum_last<real><<<592, 256, 0, c->stream>>>(R(fn), T, c->ng, st); PFAG_LAUNCHED(c);
+            }
+            if (hst[3]) c->stats.relax_failures++;
         }
-        if (iters_out) *iters_out = ri;
+        if (iters_out) *iters_out = hst[1];
         return PFAG_OK;
     }
     int normals() {
@@ -938,43 +981,60 @@ struct Plain {
         PFAG_LAUNCHED(c);
         return bc_cells(c->phin, c->Ntot);
     }
+    static constexpr int CELL_AHEAD = 8, LUM_AHEAD = 2;
+    int cell_check(int nblk, bool odd, int *active, int *ri, int *iters) {
+        const double *part = c->part_z;
+        if (c->serial_sums) {
+            const real *Q = odd ? R(c->cell_t) : R(c->phin);
+            k_serial_cell_rdev<real><<<(c->Ntot + 63) / 64, 64, 0, c->stream>>>(
+                Q, R(c->phi), odd, c->d_xc, c->d_yc, c->N, c->zone, c->Ntot, c->dp.dx, (double)c->dp.Ncur, active,
+                c->d_part);
+            PFAG_LAUNCHED(c);
+            part = c->d_part;
+            nblk = 1;
+        }
+        k_cell_check<<<c->Ntot, 32, 0, c->stream>>>(part, nblk, c->dp.thr_cells, c->p.rimax, active, ri, iters,
+                                                    c->d_err);
+        PFAG_LAUNCHED(c);
+        return PFAG_OK;
+    }
     int reshape_cells() {
         const int Nt = c->Ntot;
-        int *active = c->d_iflags, *ri = c->d_iflags + Nt, *nact = c->d_iflags + 2 * Nt;
-        // all cells start active with ri = 0
+        int *active = c->d_iflags, *ri = c->d_iflags + Nt, *iters = c->d_iflags + 2 * Nt;
+        // all cells start active with ri = 0 and no iteration done
         std::fill(c->h_iflags, c->h_iflags + Nt, 1);
-        std::fill(c->h_iflags + Nt, c->h_iflags + 2 * Nt + 1, 0);
-        PFAG_CUDA_CHECK(cudaMemcpyAsync(c->d_iflags, c->h_iflags, sizeof(int) * (2 * Nt + 1), cudaMemcpyHostToDevice,
+        std::fill(c->h_iflags + Nt, c->h_iflags + 3 * Nt, 0);
+        PFAG_CUDA_CHECK(cudaMemcpyAsync(c->d_iflags, c->h_iflags, sizeof(int) * 3 * Nt, cudaMemcpyHostToDevice,
                                         c->stream));
         const real A = (real)c->dp.A_resh, B = (real)c->dp.B_resh;
         const double scale = c->dp.dx * c->dp.dx / (double)c->dp.Ncur;
-        const int nblk = c->serial_sums ? 1 : 32;
-        for (;;) {
-            k_zone_copy<real><<<zone_grid(), dim3(TBX, TBY), 0, c->stream>>>(R(c->phi), R(c->phin), c->d_xc, c->d_yc,
-                                                                             c->N, c->zone, active);
-            PFAG_LAUNCHED(c);
-            k_cell_relax<real><<<zone_grid(), dim3(TBX, TBY), 0, c->stream>>>(
-                R(c->phi), R(c->phin), R(c->jx), R(c->jy), c->d_xc, c->d_yc, c->N, c->zone, A, B, active);
-            PFAG_LAUNCHED(c);
-            if (c->serial_sums)
-                k_serial_cell_rdev<real><<<(Nt + 63) / 64, 64, 0, c->stream>>>(
-                    R(c->phin), R(c->phi), c->d_xc, c->d_yc, c->N, c->zone, Nt, c->dp.dx, (double)c->dp.Ncur, active,
-                    c->d_part);
-            else
-                k_cell_rdev<real><<<dim3(nblk, Nt), RED_THREADS, 0, c->stream>>>(
-                    R(c->phin), R(c->phi), c->d_xc, c->d_yc, c->N, c->zone, scale, active, c->d_part);
-            PFAG_LAUNCHED(c);
-            PFAG_CUDA_CHECK(cudaMemsetAsync(nact, 0, sizeof(int), c->stream));
-            k_cell_check<<<(Nt + 127) / 128, 128, 0, c->stream>>>(c->d_part, nblk, Nt, c->dp.thr_cells, c->p.rimax,
-                                                                   active, ri, nact, c->d_err);
-            PFAG_LAUNCHED(c);
-            PFAG_CUDA_CHECK(cudaMemcpyAsync(c->h_iflags + 2 * Nt, nact, sizeof(int), cudaMemcpyDeviceToHost,
+        const dim3 g = zone_grid();
+        const int nblk = (int)(g.x * g.y);
+        real *T = R(c->cell_t);
+        // CELL_AHEAD iterations enqueued between the host's looks at the flags: a
+        // look costs a copy and a wait, an iteration of stopped cells two launches
+        // that return (7 cells, 17 iterations: 38 us an iteration with five
+        // launches and a look each, PLAIN_NEW)
+        for (bool any = true; any;) {
+            for (int k = 0; k < CELL_AHEAD; k += 2) {
+                k_cell_iter<real, true><<<g, 256, 0, c->stream>>>(R(c->phi), R(c->phin), T, R(c->jx), R(c->jy), c->d_xc,
+                                                                 c->d_yc, c->N, c->zone, A, B, scale, active, c->part_z);
+                PFAG_LAUNCHED(c);
+                PFAG_TRY(cell_check(nblk, true, active, ri, iters));
+                k_cell_iter<real, false><<<g, 256, 0, c->stream>>>(R(c->phi), R(c->phin), T, R(c->jx), R(c->jy),
+                                                                  c->d_xc, c->d_yc, c->N, c->zone, A, B, scale, active,
+                                                                  c->part_z);
+                PFAG_LAUNCHED(c);
+                PFAG_TRY(cell_check(nblk, false, active, ri, iters));
+            }
+            PFAG_CUDA_CHECK(cudaMemcpyAsync(c->h_iflags, c->d_iflags, sizeof(int) * 2 * Nt, cudaMemcpyDeviceToHost,
                                             c->stream));
             PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
-            if (c->h_iflags[2 * Nt] == 0) break;
+            any = false;
+            for (int n = 0; n < Nt; n++) any = any || c->h_iflags[n];
         }
-        PFAG_CUDA_CHECK(cudaMemcpyAsync(c->h_iflags + Nt, ri, sizeof(int) * Nt, cudaMemcpyDeviceToHost, c->stream));
-        PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
+        k_cell_last<real><<<g, 256, 0, c->stream>>>(R(c->phin), T, c->d_xc, c->d_yc, c->N, c->zone, iters);
+        PFAG_LAUNCHED(c);
         int mx = 0, sm = 0;
         for (int n = 0; n < Nt; n++) {
             // the loop body increments ri once per iteration that does not break
@@ -1069,6 +1129,12 @@ int pfag_plain_alloc(pfag_ctx *c) {
     PFAG_CUDA_CHECK(cudaMalloc(&c->jx, nc * rs));
     PFAG_CUDA_CHECK(cudaMalloc(&c->jy, nc * rs));
     PFAG_CUDA_CHECK(cudaMalloc(&c->ngl, ng * rs));
+    const size_t Z = 2 * (size_t)c->zone;
+    PFAG_CUDA_CHECK(cudaMalloc(&c->cell_t, c->Ntot * Z * Z * rs));
+    PFAG_CUDA_CHECK(cudaMalloc(&c->lum_t, ng * rs));
+    const size_t zb = c->Ntot * ((Z + TBX - 1) / TBX) * ((Z + TBY - 1) / TBY);
+    const size_t lb = (size_t)((c->N + TBX - 1) / TBX) * ((c->N + TBY - 1) / TBY);
+    PFAG_CUDA_CHECK(cudaMalloc(&c->part_z, std::max(zb, lb) * sizeof(double)));
     for (int k = 0; k < 6; k++) PFAG_CUDA_CHECK(cudaMalloc(&c->maps[k], nc * rs));
     PFAG_CUDA_CHECK(cudaMalloc(&c->pixx, nc * rs));
     PFAG_CUDA_CHECK(cudaMalloc(&c->pixy, nc * rs));
@@ -1087,7 +1153,8 @@ int pfag_plain_alloc(pfag_ctx *c) {
 }
 
 void pfag_plain_free(pfag_ctx *c) {
-    void *bufs[] = {c->g, c->pnd, c->jx, c->jy, c->ngl, c->pixx, c->pixy, c->piyy, c->fftbuf};
+    void *bufs[] = {c->g, c->pnd, c->jx, c->jy, c->ngl, c->pixx, c->pixy, c->piyy, c->fftbuf, c->cell_t, c->lum_t,
+                    c->part_z};
     for (void *b : bufs) if (b) cudaFree(b);
     for (int k = 0; k < 6; k++) if (c->maps[k]) cudaFree(c->maps[k]);
     if (c->plan_ok) cufftDestroy(c->plan);
