@@ -1226,7 +1226,7 @@ __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 4 : 2) kr_boxD2(const
 }
 
 template <typename real, int M, int G, int BT>
-__global__ void __launch_bounds__(BT, 1280 / BT) kr_boxB(typename Cplx<real>::type *__restrict__ Y1,
+__global__ void __launch_bounds__(BT, (sizeof(real) == 4 ? 1280 : 512) / BT) kr_boxB(typename Cplx<real>::type *__restrict__ Y1,
                                                const typename Cplx<real>::type *__restrict__ Y2,
                                                const unsigned char *__restrict__ clsT, BoxArgs a) {
     typedef typename Cplx<real>::type cx;

@@ -89,6 +89,7 @@ struct pfag_ctx {
     void *fftbuf;   // 11 * Ntot * M*M complex
     void *cell_t, *lum_t;   // the plain loops' second iterate: [Ntot][2z][2z], [N][N]
     double *part_z;         // their blocks' sums
+    void *plain_graphs;     // the plain step's captured stretches (pfag_plain.cu)
     cufftHandle plan;
     bool plan_ok;
     // small device arrays

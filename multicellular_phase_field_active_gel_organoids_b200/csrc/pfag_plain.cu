@@ -519,6 +519,10 @@ __global__ void k_lum_iter(const real *__restrict__ p, real *__restrict__ q, rea
     if (threadIdx.x == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = r;
 }
 
+__global__ void k_lum_state(int *st, int active) {
+    if (threadIdx.x < 4) st[threadIdx.x] = threadIdx.x == 0 ? active : 0;
+}
+
 // The loop's end test after it (:851-868): rdev from the blocks' sums in a fixed
 // order.  st: [0] active, [1] ri, [2] iterations, [3] passed rimax.
 __global__ void k_lum_check(const double *__restrict__ part, int npart, double thr, int rimax, int *__restrict__ st) {
@@ -654,6 +658,12 @@ __global__ void k_cell_last(real *__restrict__ phin, const real *__restrict__ T,
             T[(size_t)n * Z * Z + (size_t)li * Z + lj];
 }
 
+// all cells active with ri = 0 and no iteration done ([3][ncells])
+__global__ void k_cell_state(int *st, int ncells) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 3 * ncells; k += gridDim.x * blockDim.x)
+        st[k] = k < ncells ? 1 : 0;
+}
+
 // Convergence bookkeeping of the while loop at cell_phase_functions.cpp:475-574:
 // after an iteration, the loop ends when rdev <= thr, or (ri > rimax) breaks.
 // One warp per cell; rdev from the blocks' sums in a fixed order.
@@ -765,6 +775,21 @@ template <> struct FFTX<float> {
         return cufftExecC2C(p, (cufftComplex *)in, (cufftComplex *)out, dir);
     }
     static constexpr cufftType type = CUFFT_C2C;
+};
+
+// the step's captured stretches (Plain::stretch)
+struct PlainGraphs {
+    cudaGraphExec_t exec[5] = {};
+    long launches[5] = {};
+    long steps = 0;            // steps taken: the first one runs eagerly
+    bool failed = false;       // a refused capture: eager from then on
+    int key = 0;
+    void drop() {
+        for (cudaGraphExec_t &e : exec) {
+            if (e) cudaGraphExecDestroy(e);
+            e = nullptr;
+        }
+    }
 };
 
 template <typename real>
@@ -914,10 +939,12 @@ struct Plain {
         PFAG_LAUNCHED(c);
         return PFAG_OK;
     }
-    int reshape_lum(int which, int *iters_out) {
+    // the lumen's (which 0) or the ECM's relaxation: normals and the loop's state
+    // on the device (active, ri, iterations, passed rimax)
+    int *lum_state() { return c->d_iflags + 8 * c->Ntot; }
+    int lum_begin(int which) {
         const int N = c->N;
         void *f = which ? c->ecm : c->lum, *fn = which ? c->ecmn : c->lumn;
-        const real side = which ? (real)1.0 : (real)0.0;
         k_norm_grad_2d<real><<<interior_grid(1), dim3(TBX, TBY), 0, c->stream>>>(R(f), R(c->ngl), N, c4());
         PFAG_LAUNCHED(c);
         PFAG_TRY(bc_cells(c->ngl, 1));
@@ -927,45 +954,60 @@ struct Plain {
         PFAG_LAUNCHED(c);
         PFAG_TRY(bc_cells(c->jx, 1));
         PFAG_TRY(bc_cells(c->jy, 1));
-        // the loop's state on the device: active, ri, iterations, passed rimax; the
-        // host looks at it after LUM_AHEAD iterations enqueued (the ones past
-        // the end do nothing)
-        int *st = c->d_iflags + 8 * c->Ntot, *hst = c->h_iflags + 8 * c->Ntot;
-        hst[0] = c->dp.rdev0_lum > c->dp.thr_lum ? 1 : 0;
-        hst[1] = hst[2] = hst[3] = 0;
-        if (hst[0]) {
-            const real A = (real)c->dp.A_resh, B = (real)c->dp.B_resh;
-            const dim3 g((N + TBX - 1) / TBX, (N + TBY - 1) / TBY);
-            real *T = R(c->lum_t);
-            PFAG_CUDA_CHECK(cudaMemcpyAsync(st, hst, 4 * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-            const int ahead = c->serial_sums ? 1 : LUM_AHEAD;
-            for (int it = 1; hst[0];) {
-                for (int k = 0; k < ahead; k++, it++) {
-                    real *P = (it & 1) ? R(fn) : T, *Q = (it & 1) ? T : R(fn);
-                    k_lum_iter<real><<<g, 256, 0, c->stream>>>(P, Q, R(f), R(c->jx), R(c->jy), N, A, B, side,
-                                                               c->dp.dx * c->dp.dx, st, c->part_z);
-                    PFAG_LAUNCHED(c);
-                    const double *part = c->part_z;
-                    int npart = (int)(g.x * g.y);
-                    if (c->serial_sums) {
-                        k_serial_absdiff<real><<<1, 32, 0, c->stream>>>(Q, R(f), N, c->dp.dx, c->d_scal + 1);
-                        PFAG_LAUNCHED(c);
-                        part = c->d_scal + 1;
-                        npart = 1;
-                    }
-                    k_lum_check<<<1, RED_THREADS, 0, c->stream>>>(part, npart, c->dp.thr_lum, c->p.rimax, st);
-                    PFAG_LAUNCHED(c);
-                }
-                PFAG_CUDA_CHECK(cudaMemcpyAsync(hst, st, 4 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-                PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
+        k_lum_state<<<1, 32, 0, c->stream>>>(lum_state(), c->dp.rdev0_lum > c->dp.thr_lum ? 1 : 0);
+        PFAG_LAUNCHED(c);
+        return PFAG_OK;
+    }
+    // iterations it .. it + count - 1, then the state on its way to the host
+    int lum_iters(int which, int it, int count) {
+        const int N = c->N;
+        void *f = which ? c->ecm : c->lum, *fn = which ? c->ecmn : c->lumn;
+        const real side = which ? (real)1.0 : (real)0.0;
+        const real A = (real)c->dp.A_resh, B = (real)c->dp.B_resh;
+        const dim3 g((N + TBX - 1) / TBX, (N + TBY - 1) / TBY);
+        real *T = R(c->lum_t);
+        int *st = lum_state();
+        for (int k = 0; k < count; k++, it++) {
+            real *P = (it & 1) ? R(fn) : T, *Q = (it & 1) ? T : R(fn);
+            k_lum_iter<real><<<g, 256, 0, c->stream>>>(P, Q, R(f), R(c->jx), R(c->jy), N, A, B, side,
+                                                       c->dp.dx * c->dp.dx, st, c->part_z);
+            PFAG_LAUNCHED(c);
+            const double *part = c->part_z;
+            int npart = (int)(g.x * g.y);
+            if (c->serial_sums) {
+                k_serial_absdiff<real><<<1, 32, 0, c->stream>>>(Q, R(f), N, c->dp.dx, c->d_scal + 1);
+                PFAG_LAUNCHED(c);
+                part = c->d_scal + 1;
+                npart = 1;
             }
-            if (hst[2] & 1) {
-                k_lum_last<real><<<592, 256, 0, c->stream>>>(R(fn), T, c->ng, st); PFAG_LAUNCHED(c);
-            }
-            if (hst[3]) c->stats.relax_failures++;
+            k_lum_check<<<1, RED_THREADS, 0, c->stream>>>(part, npart, c->dp.thr_lum, c->p.rimax, st);
+            PFAG_LAUNCHED(c);
         }
+        PFAG_CUDA_CHECK(cudaMemcpyAsync(c->h_iflags + 8 * c->Ntot, st, 4 * sizeof(int), cudaMemcpyDeviceToHost,
+                                        c->stream));
+        return PFAG_OK;
+    }
+    // after the first LUM_AHEAD iterations: the host looks at the state, enqueues
+    // more while the loop runs (iterations past its end do nothing)
+    int lum_finish(int which, int *iters_out) {
+        int *hst = c->h_iflags + 8 * c->Ntot;
+        PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
+        for (int it = LUM_AHEAD + 1; hst[0]; it += LUM_AHEAD) {
+            PFAG_TRY(lum_iters(which, it, LUM_AHEAD));
+            PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
+        }
+        if (hst[2] & 1) {
+            k_lum_last<real><<<592, 256, 0, c->stream>>>(R(which ? c->ecmn : c->lumn), R(c->lum_t), c->ng, lum_state());
+            PFAG_LAUNCHED(c);
+        }
+        if (hst[3]) c->stats.relax_failures++;
         if (iters_out) *iters_out = hst[1];
         return PFAG_OK;
+    }
+    int reshape_lum(int which, int *iters_out) {
+        PFAG_TRY(lum_begin(which));
+        PFAG_TRY(lum_iters(which, 1, LUM_AHEAD));
+        return lum_finish(which, iters_out);
     }
     int normals() {
         k_normals<real><<<interior_grid(c->Ntot), dim3(TBX, TBY), 0, c->stream>>>(
@@ -998,43 +1040,61 @@ struct Plain {
         PFAG_LAUNCHED(c);
         return PFAG_OK;
     }
-    int reshape_cells() {
+    int cells_begin() {
+        k_cell_state<<<4, 256, 0, c->stream>>>(c->d_iflags, c->Ntot);
+        PFAG_LAUNCHED(c);
+        return PFAG_OK;
+    }
+    // CELL_AHEAD iterations, then the flags on their way to the host: a look costs
+    // a copy and a wait, an iteration of stopped cells two launches that return
+    // (7 cells of 130 x 130, 17 iterations a step, double: 1255 us a step with five
+    // launches and a look per iteration, 693 so)
+    int cells_iters() {
         const int Nt = c->Ntot;
-        int *active = c->d_iflags, *ri = c->d_iflags + Nt, *iters = c->d_iflags + 2 * Nt;
-        // all cells start active with ri = 0 and no iteration done
-        std::fill(c->h_iflags, c->h_iflags + Nt, 1);
-        std::fill(c->h_iflags + Nt, c->h_iflags + 3 * Nt, 0);
-        PFAG_CUDA_CHECK(cudaMemcpyAsync(c->d_iflags, c->h_iflags, sizeof(int) * 3 * Nt, cudaMemcpyHostToDevice,
-                                        c->stream));
+        int *active = c->d_iflags, *ri = active + Nt, *iters = active + 2 * Nt;
         const real A = (real)c->dp.A_resh, B = (real)c->dp.B_resh;
         const double scale = c->dp.dx * c->dp.dx / (double)c->dp.Ncur;
         const dim3 g = zone_grid();
         const int nblk = (int)(g.x * g.y);
         real *T = R(c->cell_t);
-        // CELL_AHEAD iterations enqueued between the host's looks at the flags: a
-        // look costs a copy and a wait, an iteration of stopped cells two launches
-        // that return (7 cells, 17 iterations: 38 us an iteration with five
-        // launches and a look each, PLAIN_NEW)
-        for (bool any = true; any;) {
-            for (int k = 0; k < CELL_AHEAD; k += 2) {
-                k_cell_iter<real, true><<<g, 256, 0, c->stream>>>(R(c->phi), R(c->phin), T, R(c->jx), R(c->jy), c->d_xc,
-                                                                 c->d_yc, c->N, c->zone, A, B, scale, active, c->part_z);
-                PFAG_LAUNCHED(c);
-                PFAG_TRY(cell_check(nblk, true, active, ri, iters));
-                k_cell_iter<real, false><<<g, 256, 0, c->stream>>>(R(c->phi), R(c->phin), T, R(c->jx), R(c->jy),
-                                                                  c->d_xc, c->d_yc, c->N, c->zone, A, B, scale, active,
-                                                                  c->part_z);
-                PFAG_LAUNCHED(c);
-                PFAG_TRY(cell_check(nblk, false, active, ri, iters));
-            }
-            PFAG_CUDA_CHECK(cudaMemcpyAsync(c->h_iflags, c->d_iflags, sizeof(int) * 2 * Nt, cudaMemcpyDeviceToHost,
-                                            c->stream));
-            PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
-            any = false;
-            for (int n = 0; n < Nt; n++) any = any || c->h_iflags[n];
+        for (int k = 0; k < CELL_AHEAD; k += 2) {
+            k_cell_iter<real, true><<<g, 256, 0, c->stream>>>(R(c->phi), R(c->phin), T, R(c->jx), R(c->jy), c->d_xc,
+                                                             c->d_yc, c->N, c->zone, A, B, scale, active, c->part_z);
+            PFAG_LAUNCHED(c);
+            PFAG_TRY(cell_check(nblk, true, active, ri, iters));
+            k_cell_iter<real, false><<<g, 256, 0, c->stream>>>(R(c->phi), R(c->phin), T, R(c->jx), R(c->jy), c->d_xc,
+                                                              c->d_yc, c->N, c->zone, A, B, scale, active, c->part_z);
+            PFAG_LAUNCHED(c);
+            PFAG_TRY(cell_check(nblk, false, active, ri, iters));
         }
-        k_cell_last<real><<<g, 256, 0, c->stream>>>(R(c->phin), T, c->d_xc, c->d_yc, c->N, c->zone, iters);
+        PFAG_CUDA_CHECK(cudaMemcpyAsync(c->h_iflags, c->d_iflags, sizeof(int) * 2 * Nt, cudaMemcpyDeviceToHost,
+                                        c->stream));
+        return PFAG_OK;
+    }
+    int cells_last() {
+        k_cell_last<real><<<zone_grid(), 256, 0, c->stream>>>(R(c->phin), R(c->cell_t), c->d_xc, c->d_yc, c->N, c->zone,
+                                                              c->d_iflags + 2 * c->Ntot);
         PFAG_LAUNCHED(c);
+        return PFAG_OK;
+    }
+    // waits for the flags; whether some cell still iterates
+    int cells_look(bool *any) {
+        PFAG_CUDA_CHECK(cudaStreamSynchronize(c->stream));
+        *any = false;
+        for (int n = 0; n < c->Ntot; n++) *any = *any || c->h_iflags[n];
+        return PFAG_OK;
+    }
+    int reshape_cells() {
+        PFAG_TRY(cells_begin());
+        for (bool any = true; any;) {
+            PFAG_TRY(cells_iters());
+            PFAG_TRY(cells_look(&any));
+        }
+        PFAG_TRY(cells_last());
+        return cells_stats();
+    }
+    int cells_stats() {
+        const int Nt = c->Ntot;
         int mx = 0, sm = 0;
         for (int n = 0; n < Nt; n++) {
             // the loop body increments ri once per iteration that does not break
@@ -1097,26 +1157,84 @@ struct Plain {
         PFAG_CUDA_CHECK(cudaStreamSynchronize(s));
         return pfag_check_device_error(c);
     }
+    // One stretch of the step without a look of the host: enqueued by f, and from
+    // the second step on replayed as a CUDA graph (about 100 launches of a step
+    // in five graphs: 7 cells of 130 x 130, 693 us a step with single launches,
+    // 474 so).
+    template <typename Fn> int stretch(int k, Fn f) {
+        PlainGraphs *pg = (PlainGraphs *)c->plain_graphs;
+        if (!pg || pg->steps < 1 || pg->failed || pfag_prof_on(c)) return f();
+        if (!pg->exec[k]) {
+            const long l0 = c->launches;
+            pg->failed = true;
+            if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+                const int rc = f();
+                cudaGraph_t g = nullptr;
+                const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+                if (rc == PFAG_OK && e == cudaSuccess && g && cudaGraphInstantiate(&pg->exec[k], g, 0) == cudaSuccess) {
+                    pg->failed = false;
+                    pg->launches[k] = c->launches - l0;
+                } else {
+                    pg->exec[k] = nullptr;
+                }
+                if (g) cudaGraphDestroy(g);
+            }
+            c->launches = l0;
+            (void)cudaGetLastError();
+            if (pg->failed) return f();
+        }
+        PFAG_CUDA_CHECK(cudaGraphLaunch(pg->exec[k], c->stream));
+        c->launches += pg->launches[k];
+        return PFAG_OK;
+    }
     int step(int it) {
         (void)it;
+        PlainGraphs *pg = (PlainGraphs *)c->plain_graphs;
+        // the captured launches depend on these two switches
+        const int key = (c->serial_sums ? 1 : 0) | (c->debug ? 2 : 0);
+        if (pg && pg->key != key) {
+            pg->drop();
+            pg->key = key;
+        }
         PFAG_TRY(centres());
         PFAG_TRY(check_zone());
-        PFAG_TRY(maps());
-        PFAG_TRY(hfunc3d());
-        PFAG_TRY(hfunc2d());
-        PFAG_TRY(norm_grad());
-        PFAG_TRY(prod_norm_delta());
-        PFAG_TRY(psi());
-        PFAG_TRY(sum_s());
-        PFAG_TRY(cortices());
-        PFAG_TRY(lum_ecm_update());
-        PFAG_TRY(reshape_lum(0, &c->stats.lum_iters));
-        PFAG_TRY(reshape_lum(1, &c->stats.ecm_iters));
-        PFAG_TRY(normals());
-        PFAG_TRY(update_cells());
-        PFAG_TRY(reshape_cells());
-        PFAG_TRY(copy_back());
-        return PFAG_OK;
+        PFAG_TRY(stretch(0, [&] {
+            PFAG_TRY(maps());
+            PFAG_TRY(hfunc3d());
+            PFAG_TRY(hfunc2d());
+            PFAG_TRY(norm_grad());
+            PFAG_TRY(prod_norm_delta());
+            PFAG_TRY(psi());
+            PFAG_TRY(sum_s());
+            PFAG_TRY(cortices());
+            PFAG_TRY(lum_ecm_update());
+            PFAG_TRY(lum_begin(0));
+            return lum_iters(0, 1, LUM_AHEAD);
+        }));
+        PFAG_TRY(lum_finish(0, &c->stats.lum_iters));
+        PFAG_TRY(stretch(1, [&] {
+            PFAG_TRY(lum_begin(1));
+            return lum_iters(1, 1, LUM_AHEAD);
+        }));
+        PFAG_TRY(lum_finish(1, &c->stats.ecm_iters));
+        PFAG_TRY(stretch(2, [&] {
+            PFAG_TRY(normals());
+            PFAG_TRY(update_cells());
+            PFAG_TRY(cells_begin());
+            return cells_iters();
+        }));
+        bool any = false;
+        PFAG_TRY(cells_look(&any));
+        while (any) {
+            PFAG_TRY(stretch(3, [&] { return cells_iters(); }));
+            PFAG_TRY(cells_look(&any));
+        }
+        PFAG_TRY(stretch(4, [&] {
+            PFAG_TRY(cells_last());
+            return copy_back();
+        }));
+        if (pg) pg->steps++;
+        return cells_stats();
     }
 };
 
@@ -1149,10 +1267,16 @@ int pfag_plain_alloc(pfag_ctx *c) {
                                    c->prec == 64 ? CUFFT_Z2Z : CUFFT_C2C, c->Ntot));
     PFAG_CUFFT_CHECK(cufftSetStream(c->plan, c->stream));
     c->plan_ok = true;
+    c->plain_graphs = new PlainGraphs();
     return PFAG_OK;
 }
 
 void pfag_plain_free(pfag_ctx *c) {
+    if (PlainGraphs *pg = (PlainGraphs *)c->plain_graphs) {
+        pg->drop();
+        delete pg;
+        c->plain_graphs = nullptr;
+    }
     void *bufs[] = {c->g, c->pnd, c->jx, c->jy, c->ngl, c->pixx, c->pixy, c->piyy, c->fftbuf, c->cell_t, c->lum_t,
                     c->part_z};
     for (void *b : bufs) if (b) cudaFree(b);
