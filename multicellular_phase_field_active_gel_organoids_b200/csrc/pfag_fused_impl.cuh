@@ -121,6 +121,7 @@ struct FusedRes {
     cudaEvent_t ev_upd, ev_spec;
     bool split;             // this organoid's steps run them so
     int npsi;
+    int nsm;                // the device's SMs
     int coop_r;             // co-resident block count of the persistent cells kernel
     int coop_default;       // its value before any launch-shape setting
     int coop_l, coop_l_default;   // the same of the persistent lumen / ECM kernel
@@ -883,15 +884,27 @@ __device__ __forceinline__ void box_stress(const BoxArgs &a, real f, real dxp, r
 }
 
 // ---- box passes on register-resident FFTs (M = 32 .. 256) ----------------
-template <int M> struct BoxGeom {
+// Blocks of BT threads: 256, or 64 where 256 would leave SMs without a block
+// (Fused::box_reg).
+template <int M, int BT = 256> struct BoxGeom {
     static constexpr int TT = RegFFT<float2, M>::TT;          // threads per transform
-    static constexpr int ROWS = (256 / TT < M) ? 256 / TT : M; // rows per block of the row passes
+    static constexpr int ROWS = (BT / TT < M) ? BT / TT : M;   // rows per block of the row passes
     static constexpr int THREADS = TT * ROWS;
     static constexpr int WG = 32 / TT;                       // thread groups per warp
 };
 
-// Pass A on register FFTs: one thread group per box row.
-template <typename real, int M>
+// Pass A on register FFTs: one thread group per box row.  BT = 64: four times
+// the threads of the block's thread groups form the stresses and hand them over
+// in shared memory (a chain of ten divisions and an exponential per element in
+// FP64 is what bounds a block: 7 cells of 128 x 128 in a step's event times, of
+// which about 6.5 us are the events', FP32 14.8 -> 10.7 us, FP64 42.6 -> 18.7).
+template <typename real, int M, int BT> struct BoxA {
+    static constexpr int ROWS = BoxGeom<M, BT>::ROWS, FFT = BoxGeom<M, BT>::THREADS;
+    static constexpr int SPLIT = BT == 64 ? 4 : 1, THREADS = FFT * SPLIT;
+    static constexpr size_t smem = (M + (size_t)ROWS * M * (SPLIT > 1 ? 2 : 1)) * 2 * sizeof(real) +
+                                   (size_t)ROWS * M * sizeof(real) + (size_t)ROWS * (M + 4);
+};
+template <typename real, int M, int BT>
 __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 4 : 2) kr_boxA(const real *__restrict__ phi, const real *__restrict__ rho,
                                                const real *__restrict__ lum, const real *__restrict__ ecm,
                                                const int *__restrict__ xc, const int *__restrict__ yc, BoxArgs a,
@@ -900,11 +913,13 @@ __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 4 : 2) kr_boxA(const 
                                                unsigned char *__restrict__ clsT) {
     typedef typename Cplx<real>::type cx;
     typedef RegFFT<cx, M> RF;
-    constexpr int TT = RF::TT, E1 = RF::E1, ROWS = BoxGeom<M>::ROWS;
+    constexpr int TT = RF::TT, E1 = RF::E1, ROWS = BoxGeom<M, BT>::ROWS;
     extern __shared__ unsigned char smraw[];
     cx *tw = (cx *)smraw;
     cx *scr = tw + M;                                   // [ROWS][M] exchange scratch
-    real *xys = (real *)(scr + ROWS * M);               // [ROWS][M] pi_xy, read back by the same thread
+    constexpr int FFT = BoxA<real, M, BT>::FFT, SPLIT = BoxA<real, M, BT>::SPLIT;
+    cx *str = scr + ROWS * M;                           // SPLIT: [ROWS][M] pi_xx + i pi_yy
+    real *xys = (real *)(str + (SPLIT > 1 ? ROWS * M : 0));  // [ROWS][M] pi_xy
     unsigned char *cls = (unsigned char *)(xys + ROWS * M);  // [ROWS][M + 4]: padded against bank conflicts
     const int t = threadIdx.x % TT, g = threadIdx.x / TT;
     const int n = blockIdx.y, i0 = blockIdx.x * ROWS, i = i0 + g;
@@ -938,53 +953,71 @@ __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 4 : 2) kr_boxA(const 
     __syncthreads();
     const size_t rowo = ((size_t)n * M + i) * M;
     cx v[E1];
-#pragma unroll
-    for (int q = 0; q < E1; q++) {
-        const int j = RF::in_index(t, q);
-        const size_t s = (size_t)(bi + i) * N + (bj + j);
-        const int o = (g + 1) * PW + j + 1;
+    // row w of the block, box column j; returns pi_xx + i pi_yy
+    auto stress = [&](int w, int j) {
+        const size_t s = (size_t)(bi + i0 + w) * N + (bj + j);
+        const int o = (w + 1) * PW + j + 1;
         const real f = sphi[o];
         const real dxp = sphi[o + PW] - sphi[o - PW];
         const real dyp = sphi[o + 1] - sphi[o - 1];
         real xx, yy, xy, rt;
         int c;
-        box_stress<real>(a, f, dxp, dyp, xys[g * M + j], lum[s], ecm[s], p1[s], p2[s], xx, yy, xy, rt, c);
-        Rb[rowo + j] = rt;
-        cls[g * (M + 4) + j] = (unsigned char)c;
-        xys[g * M + j] = xy;
-        v[q].x = xx;
-        v[q].y = yy;
+        box_stress<real>(a, f, dxp, dyp, xys[w * M + j], lum[s], ecm[s], p1[s], p2[s], xx, yy, xy, rt, c);
+        Rb[((size_t)n * M + i0 + w) * M + j] = rt;
+        cls[w * (M + 4) + j] = (unsigned char)c;
+        xys[w * M + j] = xy;
+        cx r;
+        r.x = xx;
+        r.y = yy;
+        return r;
+    };
+    if constexpr (SPLIT > 1) {
+#pragma unroll 2
+        for (int e = threadIdx.x; e < ROWS * M; e += FFT * SPLIT) str[e] = stress(e / M, e % M);
+    } else {
+#pragma unroll
+        for (int q = 0; q < E1; q++) v[q] = stress(g, RF::in_index(t, q));
     }
     __syncthreads();    // every group is done with the staged phi before scr becomes exchange space
-    RF::template run<false, true>(v, t, scr + g * M, tw);
+    if (SPLIT == 1 || threadIdx.x < FFT) {
+        if constexpr (SPLIT > 1) {
 #pragma unroll
-    for (int r = 0; r < RF::R2; r++)
+            for (int q = 0; q < E1; q++) v[q] = str[g * M + RF::in_index(t, q)];
+        }
+        RF::template run<false, true>(v, t, scr + g * M, tw);
 #pragma unroll
-        for (int k2 = 0; k2 < TT; k2++) Y1[rowo + RF::out_index(t, r, k2)] = v[r * TT + k2];
+        for (int r = 0; r < RF::R2; r++)
 #pragma unroll
-    for (int q = 0; q < E1; q++) {
-        v[q].x = xys[g * M + RF::in_index(t, q)];
-        v[q].y = (real)0.0;
+            for (int k2 = 0; k2 < TT; k2++) Y1[rowo + RF::out_index(t, r, k2)] = v[r * TT + k2];
+#pragma unroll
+        for (int q = 0; q < E1; q++) {
+            v[q].x = xys[g * M + RF::in_index(t, q)];
+            v[q].y = (real)0.0;
+        }
+        RF::template run<false, true>(v, t, scr + g * M, tw);
+#pragma unroll
+        for (int r = 0; r < RF::R2; r++)
+#pragma unroll
+            for (int k2 = 0; k2 < TT; k2++) Y2[rowo + RF::out_index(t, r, k2)] = v[r * TT + k2];
     }
-    RF::template run<false, true>(v, t, scr + g * M, tw);
-#pragma unroll
-    for (int r = 0; r < RF::R2; r++)
-#pragma unroll
-        for (int k2 = 0; k2 < TT; k2++) Y2[rowo + RF::out_index(t, r, k2)] = v[r * TT + k2];
     __syncthreads();
-    // class map transposed, ROWS consecutive bytes per column, as 16-byte
-    // stores (i0 and M are multiples of 16)
-    static_assert(ROWS % 16 == 0 && M % 16 == 0, "16-byte class-map stores");
-    for (int e = threadIdx.x; e < M * (ROWS / 16); e += blockDim.x) {
-        const int j = e / (ROWS / 16), r0 = (e - j * (ROWS / 16)) * 16;
-        unsigned w[4];
+    // class map transposed, ROWS consecutive bytes per column, as stores of W
+    // words (i0 and M are multiples of ROWS)
+    constexpr int W = ROWS >= 16 ? 4 : ROWS / 4, PC = ROWS / (4 * W);
+    static_assert(ROWS % (4 * W) == 0 && M % ROWS == 0, "whole-word class-map stores");
+    for (int e = threadIdx.x; e < M * PC; e += blockDim.x) {
+        const int j = e / PC, r0 = (e - j * PC) * (4 * W);
+        unsigned w[W];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < W; q++) {
             w[q] = 0;
 #pragma unroll
             for (int b = 0; b < 4; b++) w[q] |= (unsigned)cls[(r0 + 4 * q + b) * (M + 4) + j] << (8 * b);
         }
-        *reinterpret_cast<uint4 *>(clsT + ((size_t)n * M + j) * M + i0 + r0) = make_uint4(w[0], w[1], w[2], w[3]);
+        unsigned char *dst = clsT + ((size_t)n * M + j) * M + i0 + r0;
+        if constexpr (W == 4) *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        else if constexpr (W == 2) *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
+        else *reinterpret_cast<unsigned *>(dst) = w[0];
     }
 }
 
@@ -1062,14 +1095,14 @@ __device__ __forceinline__ void store_cols_fixed(cx *__restrict__ dstg, const cx
 // Fx is stored for pass D2, and Fy is differentiated along the row at once,
 // dt kfac Re(IFFT_j(-i jr FFT_j(Fy)))/M stored beside it.  X holds Fx, the
 // row term follows at X + Ntot M^2.
-template <typename real, int M>
-__global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 2) kr_boxC2(const typename Cplx<real>::type *__restrict__ Y1,
+template <typename real, int M, int BT>
+__global__ void __launch_bounds__(BT, (sizeof(real) == 4 ? 3 : 2) * 256 / BT) kr_boxC2(const typename Cplx<real>::type *__restrict__ Y1,
                                                real *__restrict__ X, const real *__restrict__ rho,
                                                const int *__restrict__ xc, const int *__restrict__ yc, BoxArgs a,
                                                real *__restrict__ vdx, real *__restrict__ vdy) {
     typedef typename Cplx<real>::type cx;
     typedef RegFFT<cx, M> RF;
-    constexpr int TT = RF::TT, E1 = RF::E1, ROWS = BoxGeom<M>::ROWS;
+    constexpr int TT = RF::TT, E1 = RF::E1, ROWS = BoxGeom<M, BT>::ROWS;
     extern __shared__ unsigned char smraw[];
     cx *tw = (cx *)smraw;
     cx *scr = tw + M;
@@ -1135,18 +1168,18 @@ __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 2) kr_boxC2(const
 // Pass D2 (columns): two real columns of Fx per complex transform (z = a + i b:
 // the i-derivatives of a and b come back in the real and imaginary parts),
 // then the new rho = rho + dt R + column term + row term, in place.
-template <int M> struct BoxGeomD2 {
+template <int M, int BT> struct BoxGeomD2 {
     static constexpr int TT = RegFFT<float2, M>::TT;
-    static constexpr int GROUPS = 256 / TT;
+    static constexpr int GROUPS = BT / TT;
     static constexpr int COLS = (2 * GROUPS < M) ? 2 * GROUPS : M;   // real columns per block
     static constexpr int NSQ = COLS / 2;                               // complex sequences per block
 };
-template <typename real, int M>
+template <typename real, int M, int BT>
 __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 4 : 2) kr_boxD2(const real *__restrict__ X, real *__restrict__ rho,
                                                 const real *__restrict__ Rb, const int *__restrict__ xc,
                                                 const int *__restrict__ yc, BoxArgs a) {
     typedef typename Cplx<real>::type cx;
-    constexpr int S = M + 1, NSQ = BoxGeomD2<M>::NSQ, COLS = BoxGeomD2<M>::COLS;
+    constexpr int S = M + 1, NSQ = BoxGeomD2<M, BT>::NSQ, COLS = BoxGeomD2<M, BT>::COLS;
     constexpr int WG = BoxGeom<M>::WG;
     constexpr int NSP = (NSQ % WG == 0) ? NSQ : ((NSQ + WG - 1) / WG) * WG;   // padded to whole warps
     extern __shared__ unsigned char smraw[];
@@ -2988,6 +3021,7 @@ struct Fused {
         PFAG_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kf_relax_loops<real, RESH_RB>,
                                                                        r->resh_threads, r->resh_smem));
         if (per < 1) { pfag_set_error("relaxation kernel cannot be resident with %d threads", r->resh_threads); return PFAG_E_UNSUPPORTED; }
+        r->nsm = nsm;
         r->coop_r = nsm * std::min(per, 8);
         r->tpc = (2 * c->zone + RESH_RB - 1) / RESH_RB;
         {
@@ -3647,30 +3681,41 @@ struct Fused {
         }
     }
 
+    // Blocks of a quarter of the thread groups for the row passes and D2 where
+    // the full ones would not give every SM a block (D2 keeps 256 threads for
+    // its loads and stores).  Four steps of 7 cells of 128 x 128 (28 full blocks
+    // of 148 SMs): FP32 1003 -> 822 us, FP64 1094 -> 915.  Just above a block per
+    // SM either may win (FP32 us a step, full / small: 74 cells of 64 x 64 71 /
+    // 83, 37 of 128 x 128 102 / 93, 10 of 256 x 256 227 / 218), further up the
+    // full ones do (100 of 128 x 128 172 / 174, 64 of 256 x 256 293 / 308).
     template <int MM>
     int box_reg(const BoxArgs &ba) {
-        typedef BoxGeom<MM> BG;
+        const bool small = (long)(MM / BoxGeom<MM>::ROWS) * c->Ntot < r->nsm;
+        return small ? box_reg_bt<MM, 64>(ba) : box_reg_bt<MM, 256>(ba);
+    }
+    template <int MM, int BT>
+    int box_reg_bt(const BoxArgs &ba) {
+        typedef BoxGeom<MM, BT> BG;
         cudaStream_t s = bs;
         const int Nt = c->Ntot;
         const size_t cs = sizeof(cx);
-        const size_t smA = (MM + (size_t)BG::ROWS * MM) * cs + (size_t)BG::ROWS * MM * sizeof(real) +
-                           (size_t)BG::ROWS * (MM + 4);
+        const size_t smA = BoxA<real, MM, BT>::smem;
         const size_t smC = (MM + (size_t)BG::ROWS * MM) * cs;
         const int nsB = 2 * GB;
         const int nz2 = ((GB + BG::WG - 1) / BG::WG) * BG::WG;
         const size_t smB = (MM + (size_t)(nsB + nz2) * (MM + 1)) * cs + (size_t)nsB * MM;   // + class map columns
-        PFAG_TRY(smem_at_least((const void *)kr_boxA<real, MM>, smA));
+        PFAG_TRY(smem_at_least((const void *)kr_boxA<real, MM, BT>, smA));
         PFAG_TRY(smem_at_least((const void *)kr_boxB<real, MM, GB, 256>, smB));
-        typedef BoxGeomD2<MM> BD;
+        typedef BoxGeomD2<MM, BT> BD;
         constexpr int NSP2 = (BD::NSQ % BG::WG == 0) ? BD::NSQ : ((BD::NSQ + BG::WG - 1) / BG::WG) * BG::WG;
         const size_t smD2 = (MM + (size_t)NSP2 * (MM + 1)) * cs;
-        PFAG_TRY(smem_at_least((const void *)kr_boxC2<real, MM>, smC));
-        PFAG_TRY(smem_at_least((const void *)kr_boxD2<real, MM>, smD2));
+        PFAG_TRY(smem_at_least((const void *)kr_boxC2<real, MM, BT>, smC));
+        PFAG_TRY(smem_at_least((const void *)kr_boxD2<real, MM, BT>, smD2));
         cx *Y1 = (cx *)r->Y1, *Y2 = (cx *)r->Y2;
         const dim3 grow(MM / BG::ROWS, Nt);
         pfag_prof_begin(c, "kr_boxA");
-        kr_boxA<real, MM><<<grow, BG::THREADS, smA, s>>>(R(c->phi), R(c->rho), R(c->lum), R(c->ecm), c->d_xc, c->d_yc,
-                                                          ba, Y1, Y2, R(r->Rb), r->clsT);
+        kr_boxA<real, MM, BT><<<grow, BoxA<real, MM, BT>::THREADS, smA, s>>>(
+            R(c->phi), R(c->rho), R(c->lum), R(c->ecm), c->d_xc, c->d_yc, ba, Y1, Y2, R(r->Rb), r->clsT);
         PFAG_LAUNCHED(c);
         PFAG_TRY(after_pass_a());
         pfag_prof_begin(c, "kr_boxB");
@@ -3678,13 +3723,13 @@ struct Fused {
         PFAG_LAUNCHED(c);
         real *X = (real *)r->Y2;          // pass B is done with Y2: Fx, then the row term
         pfag_prof_begin(c, "kr_boxC2");
-        kr_boxC2<real, MM><<<grow, BG::THREADS, smC, s>>>(Y1, X, R(c->rho), c->d_xc, c->d_yc, ba,
-                                                           c->debug ? R(c->d_vx) : nullptr,
-                                                           c->debug ? R(c->d_vy) : nullptr);
+        kr_boxC2<real, MM, BT><<<grow, BG::THREADS, smC, s>>>(Y1, X, R(c->rho), c->d_xc, c->d_yc, ba,
+                                                               c->debug ? R(c->d_vx) : nullptr,
+                                                               c->debug ? R(c->d_vy) : nullptr);
         PFAG_LAUNCHED(c);
         PFAG_TRY(before_new_rho());
         pfag_prof_begin(c, "kr_boxD2");
-        kr_boxD2<real, MM><<<dim3(MM / BD::COLS, Nt), 256, smD2, s>>>(X, R(c->rho), R(r->Rb), c->d_xc, c->d_yc, ba);
+        kr_boxD2<real, MM, BT><<<dim3(MM / BD::COLS, Nt), 256, smD2, s>>>(X, R(c->rho), R(r->Rb), c->d_xc, c->d_yc, ba);
         PFAG_LAUNCHED(c);
         return PFAG_OK;
     }
