@@ -102,6 +102,8 @@ struct Blue {
     typedef RegFFT<cx, L> RF;
     typedef typename CxOps<cx>::real real;
     static constexpr int TT = RF::TT, E1 = RF::E1, R2 = RF::R2;
+    // registers that can hold an index below M: L >= 2 M - 1 and both even, so M <= L / 2
+    static constexpr int EH = E1 / 2;
 
     // index held in register q of thread t (the register FFT's input order)
     static __device__ __forceinline__ int idx(int t, int q) { return t + TT * q; }
@@ -120,13 +122,15 @@ struct Blue {
 
     // length-M DFT (forward exp(-2 pi i nk/M), INV exp(+...)), unnormalised, of
     // the sequence in v (input order; entries at index >= M are ignored);
-    // the result in input order, valid below M.  sm: L complex of the
+    // the result in input order, valid below M.  Only the registers below EH
+    // are read and written: the padding's half of the first transform's first
+    // stage and of the second one's last are left out.  sm: L complex of the
     // group's own shared memory; tw: the table in shared memory.
     template <bool INV>
     static __device__ __forceinline__ void dft(cx (&v)[E1], int t, int M, cx *sm, const cx *tw,
                                                const BlueTabs<cx> &tb) {
 #pragma unroll
-        for (int q = 0; q < E1; q++) {
+        for (int q = 0; q < EH; q++) {
             const int n = idx(t, q);
             if (n < M) {
                 cx c = tb.cw[n];
@@ -136,7 +140,7 @@ struct Blue {
                 v[q] = CxOps<cx>::mk((real)0.0, (real)0.0);
             }
         }
-        RF::template run<false, true>(v, t, sm, tw);
+        RF::template run<false, true, true>(v, t, sm, tw);
 #pragma unroll
         for (int p = 0; p < E1; p++) {
             cx w = tb.wf[RF::out_index(t, p / TT, p % TT)];
@@ -147,7 +151,7 @@ struct Blue {
         RF::template run<true, true>(v, t, sm, tw);
         to_in(v);
 #pragma unroll
-        for (int q = 0; q < E1; q++) {
+        for (int q = 0; q < EH; q++) {
             const int n = idx(t, q);
             if (n < M) {
                 cx c = tb.cw[n];
@@ -162,9 +166,9 @@ struct Blue {
     static __device__ __forceinline__ void deriv(cx (&v)[E1], int t, int M, cx *sm, const cx *tw,
                                                  const BlueTabs<cx> &tb) {
 #pragma unroll
-        for (int q = 0; q < E1; q++)
+        for (int q = 0; q < EH; q++)
             if (idx(t, q) >= M) v[q] = CxOps<cx>::mk((real)0.0, (real)0.0);
-        RF::template run<false, true>(v, t, sm, tw);
+        RF::template run<false, true, true>(v, t, sm, tw);
 #pragma unroll
         for (int p = 0; p < E1; p++) {
             const real hi = tb.hdi[RF::out_index(t, p / TT, p % TT)];   // times i hi
@@ -256,7 +260,7 @@ kbl_rowsA(typename Cplx<real>::type *__restrict__ Y1, const real *__restrict__ Y
           typename Cplx<real>::type *__restrict__ Hs, int M, int Ntot, BlueTabs<typename Cplx<real>::type> tb) {
     typedef typename Cplx<real>::type cx;
     typedef Blue<cx, L> B;
-    constexpr int TT = B::TT, E1 = B::E1, GPB = BlueGeom<real, L>::GPB;
+    constexpr int TT = B::TT, E1 = B::E1, EH = B::EH, GPB = BlueGeom<real, L>::GPB;
     extern __shared__ unsigned char smraw[];
     cx *tw = (cx *)smraw;
     const int t = threadIdx.x % TT, g = threadIdx.x / TT;
@@ -280,14 +284,14 @@ kbl_rowsA(typename Cplx<real>::type *__restrict__ Y1, const real *__restrict__ Y
         if (!pair) {
             const cx *src = Y1 + ((size_t)n * M + a) * M;
 #pragma unroll
-            for (int q = 0; q < E1; q++) {
+            for (int q = 0; q < EH; q++) {
                 const int j = B::idx(t, q);
                 v[q] = (live && j < M) ? src[j] : CxOps<cx>::mk((real)0.0, (real)0.0);
             }
         } else {
             const real *ra = Y2r + ((size_t)n * M + a) * M;
 #pragma unroll
-            for (int q = 0; q < E1; q++) {
+            for (int q = 0; q < EH; q++) {
                 const int j = B::idx(t, q);
                 v[q] = (live && j < M) ? CxOps<cx>::mk(ra[j], ra[j + M]) : CxOps<cx>::mk((real)0.0, (real)0.0);
             }
@@ -297,14 +301,14 @@ kbl_rowsA(typename Cplx<real>::type *__restrict__ Y1, const real *__restrict__ Y
             if (live) {
                 cx *dst = Y1 + ((size_t)n * M + a) * M;
 #pragma unroll
-                for (int q = 0; q < E1; q++) {
+                for (int q = 0; q < EH; q++) {
                     const int j = B::idx(t, q);
                     if (j < M) dst[j] = v[q];
                 }
             }
         } else {
 #pragma unroll
-            for (int q = 0; q < E1; q++) {
+            for (int q = 0; q < EH; q++) {
                 const int j = B::idx(t, q);
                 if (j < M) sm[j] = v[q];
             }
@@ -313,7 +317,7 @@ kbl_rowsA(typename Cplx<real>::type *__restrict__ Y1, const real *__restrict__ Y
         if (pair && live) {
             cx *ha = Hs + ((size_t)n * M + a) * H, *hb = ha + H;
 #pragma unroll
-            for (int q = 0; q < E1; q++) {
+            for (int q = 0; q < EH; q++) {
                 const int k = B::idx(t, q);
                 if (k < H) {
                     const cx zk = sm[k], zm = sm[(M - k) % M];
@@ -346,7 +350,7 @@ kbl_cols(ColSet<typename Cplx<real>::type> s0, ColSet<typename Cplx<real>::type>
          BlueTabs<typename Cplx<real>::type> tb) {
     typedef typename Cplx<real>::type cx;
     typedef Blue<cx, L> B;
-    constexpr int TT = B::TT, E1 = B::E1, GPB = BlueGeom<real, L>::GPB, S = L + 1;
+    constexpr int TT = B::TT, E1 = B::E1, EH = B::EH, GPB = BlueGeom<real, L>::GPB, S = L + 1;
     extern __shared__ unsigned char smraw[];
     cx *tw = (cx *)smraw;
     cx *Z = tw + L;                       // [GPB][S]
@@ -364,9 +368,9 @@ kbl_cols(ColSet<typename Cplx<real>::type> s0, ColSet<typename Cplx<real>::type>
         const int nc = min(GPB, cs.ncol - c0);
         cx *src = cs.base + (size_t)n * cs.cell_stride + c0;
         __syncthreads();                  // the previous task's stores have read Z (and the tables are staged)
-        for (int e = threadIdx.x; e < M * nc; e += blockDim.x) {
-            const int i = e / nc, c = e - i * nc;
-            blue_cp(Z + (size_t)c * S + i, src + (size_t)i * cs.stride + c);
+        for (int e = threadIdx.x; e < M * GPB; e += blockDim.x) {
+            const int i = e / GPB, c = e % GPB;
+            if (c < nc) blue_cp(Z + (size_t)c * S + i, src + (size_t)i * cs.stride + c);
         }
         blue_cp_wait();
         __syncthreads();
@@ -374,22 +378,22 @@ kbl_cols(ColSet<typename Cplx<real>::type> s0, ColSet<typename Cplx<real>::type>
             cx *col = Z + (size_t)g * S;
             cx v[E1];
 #pragma unroll
-            for (int q = 0; q < E1; q++) {
+            for (int q = 0; q < EH; q++) {
                 const int i = B::idx(t, q);
                 v[q] = (g < nc && i < M) ? col[i] : CxOps<cx>::mk((real)0.0, (real)0.0);
             }
             __syncwarp();
             B::template dft<INV>(v, t, M, col, tw, st);
 #pragma unroll
-            for (int q = 0; q < E1; q++) {
+            for (int q = 0; q < EH; q++) {
                 const int i = B::idx(t, q);
                 if (i < M) col[i] = v[q];
             }
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < M * nc; e += blockDim.x) {
-            const int i = e / nc, c = e - i * nc;
-            src[(size_t)i * cs.stride + c] = Z[(size_t)c * S + i];
+        for (int e = threadIdx.x; e < M * GPB; e += blockDim.x) {
+            const int i = e / GPB, c = e % GPB;
+            if (c < nc) src[(size_t)i * cs.stride + c] = Z[(size_t)c * S + i];
         }
     }
 }
@@ -409,7 +413,7 @@ kbl_rowsD1(const typename Cplx<real>::type *__restrict__ Y1, real *__restrict__ 
            BlueTabs<typename Cplx<real>::type> tb, real *__restrict__ vdx, real *__restrict__ vdy) {
     typedef typename Cplx<real>::type cx;
     typedef Blue<cx, L> B;
-    constexpr int TT = B::TT, E1 = B::E1, GPB = BlueGeom<real, L>::GPB;
+    constexpr int TT = B::TT, E1 = B::E1, EH = B::EH, GPB = BlueGeom<real, L>::GPB;
     extern __shared__ unsigned char smraw[];
     cx *tw = (cx *)smraw;
     const int t = threadIdx.x % TT, g = threadIdx.x / TT;
@@ -430,7 +434,7 @@ kbl_rowsD1(const typename Cplx<real>::type *__restrict__ Y1, real *__restrict__ 
         const size_t rowo = ((size_t)n * M + i) * M;
         cx v[E1];
 #pragma unroll
-        for (int q = 0; q < E1; q++) {
+        for (int q = 0; q < EH; q++) {
             const int j = B::idx(t, q);
             v[q] = (live && j < M) ? Y1[rowo + j] : CxOps<cx>::mk((real)0.0, (real)0.0);
         }
@@ -438,7 +442,7 @@ kbl_rowsD1(const typename Cplx<real>::type *__restrict__ Y1, real *__restrict__ 
         if (live) {
             const real *rh = rho + (size_t)n * N * N + (size_t)(bi + i) * N + bj;
 #pragma unroll
-            for (int q = 0; q < E1; q++) {
+            for (int q = 0; q < EH; q++) {
                 const int j = B::idx(t, q);
                 if (j < M) {
                     const real rr = rh[j];
@@ -457,7 +461,7 @@ kbl_rowsD2(real *__restrict__ X, const real *__restrict__ Rb, double dt, int M, 
            BlueTabs<typename Cplx<real>::type> tb) {
     typedef typename Cplx<real>::type cx;
     typedef Blue<cx, L> B;
-    constexpr int TT = B::TT, E1 = B::E1, GPB = BlueGeom<real, L>::GPB;
+    constexpr int TT = B::TT, E1 = B::E1, EH = B::EH, GPB = BlueGeom<real, L>::GPB;
     extern __shared__ unsigned char smraw[];
     cx *tw = (cx *)smraw;
     const int t = threadIdx.x % TT, g = threadIdx.x / TT;
@@ -477,7 +481,7 @@ kbl_rowsD2(real *__restrict__ X, const real *__restrict__ Rb, double dt, int M, 
         real *d0 = X + (size_t)Ntot * M * M + ((size_t)n * M + i0) * M;     // Fy rows i0, i0 + 1
         cx v[E1];
 #pragma unroll
-        for (int q = 0; q < E1; q++) {
+        for (int q = 0; q < EH; q++) {
             const int j = B::idx(t, q);
             v[q] = (live && j < M) ? CxOps<cx>::mk(d0[j], d0[M + j]) : CxOps<cx>::mk((real)0.0, (real)0.0);
         }
@@ -485,7 +489,7 @@ kbl_rowsD2(real *__restrict__ X, const real *__restrict__ Rb, double dt, int M, 
         if (live) {
             const real *r0 = Rb + ((size_t)n * M + i0) * M;
 #pragma unroll
-            for (int q = 0; q < E1; q++) {
+            for (int q = 0; q < EH; q++) {
                 const int j = B::idx(t, q);
                 if (j < M) {
                     d0[j] = dtr * r0[j] + v[q].x;
@@ -503,7 +507,7 @@ __global__ void __launch_bounds__(BlueGeom<real, L>::THREADS, BlueGeom<real, L>:
 kbl_colsE(real *__restrict__ X, int M, int Ntot, BlueTabs<typename Cplx<real>::type> tb) {
     typedef typename Cplx<real>::type cx;
     typedef Blue<cx, L> B;
-    constexpr int TT = B::TT, E1 = B::E1, GPB = BlueGeom<real, L>::GPB, S = L + 1;
+    constexpr int TT = B::TT, E1 = B::E1, EH = B::EH, GPB = BlueGeom<real, L>::GPB, S = L + 1;
     extern __shared__ unsigned char smraw[];
     cx *tw = (cx *)smraw;
     cx *Z = tw + L;                       // [GPB][S]: column pairs
@@ -519,9 +523,9 @@ kbl_colsE(real *__restrict__ X, int M, int Ntot, BlueTabs<typename Cplx<real>::t
         const int p0 = b * GPB, np = min(GPB, M / 2 - p0);     // column pairs 2p, 2p+1
         cx *fx = reinterpret_cast<cx *>(X + (size_t)n * M * M);  // row i, pair p at fx[i M/2 + p]
         __syncthreads();
-        for (int e = threadIdx.x; e < M * np; e += blockDim.x) {
-            const int i = e / np, p = e - i * np;
-            blue_cp(Z + (size_t)p * S + i, fx + (size_t)i * (M / 2) + p0 + p);
+        for (int e = threadIdx.x; e < M * GPB; e += blockDim.x) {
+            const int i = e / GPB, p = e % GPB;
+            if (p < np) blue_cp(Z + (size_t)p * S + i, fx + (size_t)i * (M / 2) + p0 + p);
         }
         blue_cp_wait();
         __syncthreads();
@@ -529,22 +533,22 @@ kbl_colsE(real *__restrict__ X, int M, int Ntot, BlueTabs<typename Cplx<real>::t
             cx *col = Z + (size_t)g * S;
             cx v[E1];
 #pragma unroll
-            for (int q = 0; q < E1; q++) {
+            for (int q = 0; q < EH; q++) {
                 const int i = B::idx(t, q);
                 v[q] = (g < np && i < M) ? col[i] : CxOps<cx>::mk((real)0.0, (real)0.0);
             }
             __syncwarp();
             B::deriv(v, t, M, col, tw, st);
 #pragma unroll
-            for (int q = 0; q < E1; q++) {
+            for (int q = 0; q < EH; q++) {
                 const int i = B::idx(t, q);
                 if (i < M) col[i] = v[q];
             }
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < M * np; e += blockDim.x) {
-            const int i = e / np, p = e - i * np;
-            fx[(size_t)i * (M / 2) + p0 + p] = Z[(size_t)p * S + i];
+        for (int e = threadIdx.x; e < M * GPB; e += blockDim.x) {
+            const int i = e / GPB, p = e % GPB;
+            if (p < np) fx[(size_t)i * (M / 2) + p0 + p] = Z[(size_t)p * S + i];
         }
     }
 }

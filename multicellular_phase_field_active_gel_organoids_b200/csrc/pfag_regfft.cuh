@@ -66,7 +66,7 @@ __host__ __device__ constexpr int brev_c(int x, int bits) {
 __host__ __device__ constexpr int ilog2_c(int x) { return x <= 1 ? 0 : 1 + ilog2_c(x >> 1); }
 
 // In-register 32-point DFT, as dft_dif below with twiddles in 32nds of a turn.
-template <bool INV, typename T>
+template <bool INV, bool HALF, typename T>
 __device__ __forceinline__ void dft_dif32(T (&v)[32]) {
     typedef typename CxOps<T>::real real;
 #pragma unroll
@@ -75,9 +75,10 @@ __device__ __forceinline__ void dft_dif32(T (&v)[32]) {
         for (int blk = 0; blk < 32; blk += 2 * span) {
 #pragma unroll
             for (int j = 0; j < span; j++) {
+                const bool zero = HALF && span == 16;   // b is zero
                 const T a = v[blk + j], b = v[blk + j + span];
-                v[blk + j] = cadd(a, b);
-                const T d = csub(a, b);
+                v[blk + j] = zero ? a : cadd(a, b);
+                const T d = zero ? a : csub(a, b);
                 const int m = j * (32 / (2 * span));   // twiddle W_{2span}^j = exp(-+ 2 pi i m / 32)
                 T r;
                 if (m == 0) {
@@ -98,11 +99,12 @@ __device__ __forceinline__ void dft_dif32(T (&v)[32]) {
 }
 
 // In-register E-point DFT (E in {2,4,8,16,32}); output v[p] = X[bitrev(p)].
-template <int E, bool INV, typename T>
+// HALF: the upper half of v is zero (and not read).
+template <int E, bool INV, bool HALF = false, typename T>
 __device__ __forceinline__ void dft_dif(T (&v)[E]) {
     typedef typename CxOps<T>::real real;
     if constexpr (E == 32) {
-        dft_dif32<INV>(v);
+        dft_dif32<INV, HALF>(v);
     } else {
 #pragma unroll
     for (int span = E / 2; span >= 1; span >>= 1) {
@@ -110,9 +112,10 @@ __device__ __forceinline__ void dft_dif(T (&v)[E]) {
         for (int blk = 0; blk < E; blk += 2 * span) {
 #pragma unroll
             for (int j = 0; j < span; j++) {
+                const bool zero = HALF && span == E / 2;   // b is zero
                 const T a = v[blk + j], b = v[blk + j + span];
-                v[blk + j] = cadd(a, b);
-                const T d = csub(a, b);
+                v[blk + j] = zero ? a : cadd(a, b);
+                const T d = zero ? a : csub(a, b);
                 const int m = j * (16 / (2 * span));   // twiddle W_{2span}^j = exp(-+ 2 pi i m / 16)
                 T r;
                 if (m == 0) {
@@ -147,9 +150,10 @@ struct RegFFT {
     // sm: M complex of shared memory private to the group; tw[k] = exp(-2 pi i k / M),
     // or with KT the same values laid out as [E1][TT]: tw[k1 TT + t] = exp(-2 pi i t k1 / M)
     // (a warp's twiddle loads then hit distinct banks whatever k1 is)
-    template <bool INV, bool KT = false>
+    // HALF: the upper half of the input is zero (v[E1/2..] is not read)
+    template <bool INV, bool KT = false, bool HALF = false>
     static __device__ __forceinline__ void run(T (&v)[E1], int t, T *sm, const T *tw) {
-        dft_dif<E1, INV>(v);
+        dft_dif<E1, INV, HALF>(v);
 #pragma unroll
         for (int p = 0; p < E1; p++) {
             const int k1 = brev_c(p, ilog2_c(E1));
