@@ -264,10 +264,8 @@ def kernel_bytes(cfg, precision: int, iters: dict, ubox: int, uring: int) -> dic
         "kbl_rowsD1": box * (2 * w + w + 2 * w),
         # row derivative: reads Fy and R; writes dt R + the row term over Fy
         "kbl_rowsD2": box * 3 * w,
-        # column derivative: reads Fx, writes it differentiated
-        "kbl_colsE": box * 2 * w,
-        # the new rho: reads both terms and rho, writes rho
-        "kbl_rho": box * 4 * w,
+        # column derivative and the new rho: reads Fx, the row term and rho, writes rho
+        "kbl_colsE": box * 4 * w,
     }
     return out
 

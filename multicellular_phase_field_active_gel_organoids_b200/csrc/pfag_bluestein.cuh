@@ -501,13 +501,20 @@ kbl_rowsD2(real *__restrict__ X, const real *__restrict__ Rb, double dt, int M, 
 }
 
 // Pass E' (columns): two real columns of Fx per complex sequence, the
-// derivative along the column (dt kfac folded in) stored over Fx in plane 0.
+// derivative along the column (dt kfac folded in), and the new rho on the box:
+// rho + (dt R + row term, plane 1 of X) + column term (update_fft_rho and
+// copy_to_rhon, rho_functions.cpp:213-265, by linearity).  As two kernels the
+// column term went through memory (event times, of which about 6.5 us are the
+// events': 64 cells on boxes of 398 x 398 64 + 51 -> 112 us, 6 cells 17 + 11 ->
+// 23, 19 cells on boxes of 114 x 114 11 + 7 -> 11).
 template <typename real, int L>
 __global__ void __launch_bounds__(BlueGeom<real, L>::THREADS, BlueGeom<real, L>::MINB)
-kbl_colsE(real *__restrict__ X, int M, int Ntot, BlueTabs<typename Cplx<real>::type> tb) {
+kbl_colsE(const real *__restrict__ X, real *__restrict__ rho, const int *__restrict__ xc,
+          const int *__restrict__ yc, int N, int z, int M, int Ntot, BlueTabs<typename Cplx<real>::type> tb) {
     typedef typename Cplx<real>::type cx;
     typedef Blue<cx, L> B;
     constexpr int TT = B::TT, E1 = B::E1, EH = B::EH, GPB = BlueGeom<real, L>::GPB, S = L + 1;
+    constexpr int U = 4;                  // a thread's elements in flight
     extern __shared__ unsigned char smraw[];
     cx *tw = (cx *)smraw;
     cx *Z = tw + L;                       // [GPB][S]: column pairs
@@ -521,7 +528,9 @@ kbl_colsE(real *__restrict__ X, int M, int Ntot, BlueTabs<typename Cplx<real>::t
     for (long task = blockIdx.x; task < total; task += gridDim.x) {
         const int n = (int)(task / nblk), b = (int)(task % nblk);
         const int p0 = b * GPB, np = min(GPB, M / 2 - p0);     // column pairs 2p, 2p+1
-        cx *fx = reinterpret_cast<cx *>(X + (size_t)n * M * M);  // row i, pair p at fx[i M/2 + p]
+        const cx *fx = reinterpret_cast<const cx *>(X + (size_t)n * M * M);  // row i, pair p at fx[i M/2 + p]
+        const cx *qx = reinterpret_cast<const cx *>(X + ((size_t)Ntot + n) * M * M);
+        real *rc = rho + (size_t)n * N * N + (size_t)(xc[n] - z + 1) * N + (yc[n] - z + 1) + 2 * p0;
         __syncthreads();
         for (int e = threadIdx.x; e < M * GPB; e += blockDim.x) {
             const int i = e / GPB, p = e % GPB;
@@ -546,26 +555,26 @@ kbl_colsE(real *__restrict__ X, int M, int Ntot, BlueTabs<typename Cplx<real>::t
             }
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < M * GPB; e += blockDim.x) {
-            const int i = e / GPB, p = e % GPB;
-            if (p < np) fx[(size_t)i * (M / 2) + p0 + p] = Z[(size_t)p * S + i];
+        for (int e0 = threadIdx.x; e0 < M * GPB; e0 += U * blockDim.x) {
+            cx ro[U], q[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int e = e0 + u * blockDim.x, i = e / GPB, p = e % GPB;
+                if (i < M && p < np) {
+                    ro[u].x = rc[(size_t)i * N + 2 * p];
+                    ro[u].y = rc[(size_t)i * N + 2 * p + 1];
+                    q[u] = qx[(size_t)i * (M / 2) + p0 + p];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int e = e0 + u * blockDim.x, i = e / GPB, p = e % GPB;
+                if (i < M && p < np) {
+                    const cx d = Z[(size_t)p * S + i];
+                    rc[(size_t)i * N + 2 * p] = ro[u].x + (q[u].x + d.x);
+                    rc[(size_t)i * N + 2 * p + 1] = ro[u].y + (q[u].y + d.y);
+                }
+            }
         }
-    }
-}
-
-// The new rho on every box: rho + (dt R + row term) + column term
-// (update_fft_rho and copy_to_rhon, rho_functions.cpp:213-265, by linearity;
-// planes 1 and 0 of X)
-template <typename real>
-__global__ void kbl_rho(const real *__restrict__ X, real *__restrict__ rho, const int *__restrict__ xc,
-                        const int *__restrict__ yc, int N, int z, int M, int Ntot) {
-    const int n = blockIdx.y;
-    const int bi = xc[n] - z + 1, bj = yc[n] - z + 1;
-    const real *dxc = X + (size_t)n * M * M, *q = X + (size_t)Ntot * M * M + (size_t)n * M * M;
-    real *rc = rho + (size_t)n * N * N;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < M * M; e += gridDim.x * blockDim.x) {
-        const int i = e / M, j = e - i * M;
-        real &ro = rc[(size_t)(bi + i) * N + bj + j];
-        ro = ro + (q[e] + dxc[e]);
     }
 }

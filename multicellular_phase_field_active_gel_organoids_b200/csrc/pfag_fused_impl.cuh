@@ -27,7 +27,7 @@
 //   any other even M up to 512 (the reference's default zone_size 200 gives
 //     M = 398): Bluestein transforms over the register FFTs (pfag_bluestein.cuh;
 //     kg_stress, kbl_rowsA, kbl_colsB, kg_velocity, kbl_colsC, kbl_rowsD1/D2,
-//     kbl_colsE, kbl_rho).
+//     kbl_colsE).
 // By linearity of the transform the new rho equals Re(IFFT(FFT(rho) + dt FFT(R)
 // + D))/M^2 of the reference, without the round-trip transforms of rho and R.
 #pragma once
@@ -3654,16 +3654,14 @@ struct Fused {
                 X, R(r->Rb), c->dp.dt, M, Nt, tb);
             PFAG_LAUNCHED(c);
         }
+        PFAG_TRY(before_new_rho());
         {
             const long tasks = (long)Nt * ((M / 2 + BGm::GPB - 1) / BGm::GPB);
             pfag_prof_begin(c, "kbl_colsE");
-            kbl_colsE<real, L><<<(unsigned)tasks, BGm::THREADS, sm_colsE, s>>>(X, M, Nt, tb);
+            kbl_colsE<real, L><<<(unsigned)tasks, BGm::THREADS, sm_colsE, s>>>(X, R(c->rho), c->d_xc, c->d_yc, N, z, M,
+                                                                               Nt, tb);
             PFAG_LAUNCHED(c);
         }
-        PFAG_TRY(before_new_rho());
-        pfag_prof_begin(c, "kbl_rho");
-        kbl_rho<real><<<g, 256, 0, s>>>(X, R(c->rho), c->d_xc, c->d_yc, N, z, M, Nt);
-        PFAG_LAUNCHED(c);
         return PFAG_OK;
     }
 
