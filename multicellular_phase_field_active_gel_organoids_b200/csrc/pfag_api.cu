@@ -351,14 +351,24 @@ __global__ void k_observables(const double *__restrict__ d_s, const double *__re
     }
 }
 
-// The device's address of a pinned host buffer; null for any other memory.
-static void *mapped_address(void *p) {
-    cudaPointerAttributes at{};
-    if (!p || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return nullptr;
+// The device's address of a pinned host buffer; null for any other memory, for
+// elements that are not aligned to their size, and unless every page of the
+// buffer is pinned at consecutive device addresses (those are copied).
+static void *mapped_address(void *p, size_t elem, size_t count) {
+    const uintptr_t a = (uintptr_t)p, end = a + elem * count, page = 4096;
+    if (!p || a % elem) return nullptr;
+    char *dev = nullptr;
+    for (uintptr_t q = a; q < end; q = (q / page + 1) * page) {
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, (void *)q) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
+        if (q == a) dev = (char *)at.devicePointer;
+        else if ((char *)at.devicePointer != dev + (q - a)) return nullptr;
     }
-    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+    return dev;
 }
 
 extern "C" int pfag_observables_async(pfag_ctx *c, double *s, double *f0, int *xc, int *yc) {
@@ -367,7 +377,7 @@ extern "C" int pfag_observables_async(pfag_ctx *c, double *s, double *f0, int *x
     void *dev[4];
     bool any = false;
     for (int k = 0; k < 4; k++) {
-        dev[k] = mapped_address(host[k]);
+        dev[k] = mapped_address(host[k], k < 2 ? sizeof(double) : sizeof(int), c->Ntot);
         any = any || dev[k];
     }
     if (any) {
