@@ -595,28 +595,37 @@ __global__ void kc_adam_list(AdamList L, float lr, float b1, float b2, float eps
 // (per element it took 29 us on 16 boxes of 128^2, 7 so).
 template <int C>
 __global__ void kc_mse(const __nv_bfloat16 *__restrict__ out, const float *__restrict__ target,
-                       __nv_bfloat16 *__restrict__ dout, float *__restrict__ loss, int H, int W, int nout,
+                       __nv_bfloat16 *__restrict__ dout, float *__restrict__ loss, int B, int H, int W, int nout,
                        float scale) {
-    const int Wp = W + 2, Q = (H + 2) * Wp, b = blockIdx.y;
+    const int Wp = W + 2, Q = (H + 2) * Wp;
+    const bool vec = ((uintptr_t)dout & 15) == 0;
     float acc = 0.0f;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < Q; q += gridDim.x * blockDim.x) {
-        const int yy = q / Wp, xx = q - yy * Wp;
-        const bool in = yy >= 1 && yy <= H && xx >= 1 && xx <= W;
-        const size_t o = ((size_t)b * Q + q) * C;
-        const float *t = target + (((size_t)b * H + (in ? yy - 1 : 0)) * W + (in ? xx - 1 : 0)) * nout;
-        __align__(16) __nv_bfloat16 v[C];
+    for (int b = blockIdx.y; b < B; b += gridDim.y) {
+        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < Q; q += gridDim.x * blockDim.x) {
+            const int yy = q / Wp, xx = q - yy * Wp;
+            const bool in = yy >= 1 && yy <= H && xx >= 1 && xx <= W;
+            const size_t o = ((size_t)b * Q + q) * C;
+            const float *t = target + (((size_t)b * H + (in ? yy - 1 : 0)) * W + (in ? xx - 1 : 0)) * nout;
+            __align__(16) __nv_bfloat16 v[C];
 #pragma unroll
-        for (int ch = 0; ch < C; ch++) {
-            float g = 0.0f;
-            if (in && ch < nout) {
-                const float d = __bfloat162float(out[o + ch]) - t[ch];
-                acc += d * d;
-                g = 2.0f * d * scale;
+            for (int ch = 0; ch < C; ch++) {
+                float g = 0.0f;
+                if (in && ch < nout) {
+                    const float d = __bfloat162float(out[o + ch]) - t[ch];
+                    acc += d * d;
+                    g = 2.0f * d * scale;
+                }
+                v[ch] = __float2bfloat16_rn(g);
             }
-            v[ch] = __float2bfloat16_rn(g);
-        }
+            if (vec) {
 #pragma unroll
-        for (int h = 0; h < C / 8; h++) reinterpret_cast<uint4 *>(dout + o)[h] = reinterpret_cast<const uint4 *>(v)[h];
+                for (int h = 0; h < C / 8; h++)
+                    reinterpret_cast<uint4 *>(dout + o)[h] = reinterpret_cast<const uint4 *>(v)[h];
+            } else {
+#pragma unroll
+                for (int ch = 0; ch < C; ch++) dout[o + ch] = v[ch];
+            }
+        }
     }
     // one FP32 addition per block: thousands of small ones into the growing total
     // would lose its last bits
@@ -818,8 +827,9 @@ extern "C" int pfag_adam_list(int count, float *const *p, const float *const *g,
 extern "C" int pfag_conv_mse(const void *out, const float *target, void *dout, float *loss, int B, int H, int W,
                              int c, int nout, float scale, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
-    if (c == 16) kc_mse<16><<<dim3(std::max(1, std::min(((H + 2) * (W + 2) + 255) / 256, 296 / B)), B), 256, 0, s>>>(
-        (const __nv_bfloat16 *)out, target, (__nv_bfloat16 *)dout, loss, H, W, nout, scale);
+    const int by = std::max(1, std::min(B, 65535));
+    if (c == 16) kc_mse<16><<<dim3(std::max(1, std::min(((H + 2) * (W + 2) + 255) / 256, 296 / by)), by), 256, 0, s>>>(
+        (const __nv_bfloat16 *)out, target, (__nv_bfloat16 *)dout, loss, B, H, W, nout, scale);
     else { pfag_set_error("pfag_conv_mse: %d channels", c); return PFAG_E_UNSUPPORTED; }
     PFAG_CUDA_CHECK(cudaGetLastError());
     return PFAG_OK;

@@ -116,3 +116,27 @@ def test_adam_list_equals_single_calls():
         assert all(torch.equal(x, y) for x, y in zip(a, b))
     with pytest.raises(capi.PfagError):
         capi.check(L.pfag_adam_list(17, None, None, None, None, None, None, 1e-3, 0.9, 0.999, 1e-8, 1, None))
+
+
+@pytest.mark.parametrize("B,offset", [(2, 0), (2, 2), (2, 8), (400, 0)])
+def test_loss_gradient_addresses(B, offset):
+    """The output gradient at addresses that are not 16-byte aligned, and more
+    boxes than blocks; bounds of test_gpu_conv.py."""
+    H, W, C = 5, 6, 16
+    rng = np.random.default_rng(B + offset)
+    out = co.pad(co.bf16(rng.normal(size=(B, H, W, C))))
+    tgt = rng.normal(size=(B, H, W, 2)).astype(np.float32)
+    od, td = dev(out, torch.float32).to(torch.bfloat16), dev(tgt, torch.float32)
+    buf = torch.ones(od.numel() + 16, dtype=torch.bfloat16, device="cuda")
+    loss = torch.zeros(1, dtype=torch.float32, device="cuda")
+    dst = ctypes.c_void_p(buf.data_ptr() + offset)
+    capi.check(capi.lib().pfag_conv_mse(P(od), P(td), dst, P(loss), B, H, W, C, 2, 0.5, None))
+    torch.cuda.synchronize()
+    d = out[:, 1:-1, 1:-1, :2] - tgt
+    assert abs(float(loss.item()) - float((d * d).sum())) <= 1e-4 * float((d * d).sum())
+    h = buf.float().cpu().numpy()
+    k = offset // 2
+    g = h[k:k + od.numel()].reshape(out.shape)
+    assert np.max(np.abs(g[:, 1:-1, 1:-1, :2] - d)) <= 1e-2 * np.abs(d).max()
+    assert not np.any(g[:, 1:-1, 1:-1, 2:]) and not np.any(g[:, 0])
+    assert (h[:k] == 1).all() and (h[k + od.numel():] == 1).all()
