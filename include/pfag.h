@@ -139,10 +139,11 @@ int pfag_set_serial_sums(pfag_ctx *ctx, int on);
 int pfag_seed_organoid(pfag_ctx *ctx, const double *centres, double radius, double env_radius,
                        unsigned long long seed);
 
-/* Fused path: launch shapes of the step's persistent relaxation kernel and
+/* Fused path: launch shapes of the step's persistent relaxation kernels and
  * phi update (the knobs the batched sweep's autotuner sets).  coop_blocks > 0
- * caps the persistent kernel's grid (0: the default, every co-resident block
- * up to the loops' task count); update_warps > 0 is the warp budget the phi
+ * caps the persistent kernels' grids (0: the default, every co-resident block
+ * up to the loops' task count; the cluster form of the cells' loops has a
+ * fixed grid); update_warps > 0 is the warp budget the phi
  * update sizes its row tasks for (0: the default, one full wave of the GPU).
  * The next step recaptures its graph.  No counterpart in the reference (its
  * OpenACC runtime picks the launch shapes). */

@@ -3681,7 +3681,7 @@ struct Fused {
 
     // Blocks of a quarter of the thread groups for the row passes and D2 where
     // the full ones would not give every SM a block (D2 keeps 256 threads for
-    // its loads and stores).  Four steps of 7 cells of 128 x 128 (28 full blocks
+    // its loads and stores).  Ten steps of 7 cells of 128 x 128 (28 full blocks
     // of 148 SMs): FP32 1003 -> 822 us, FP64 1094 -> 915.  Just above a block per
     // SM either may win (FP32 us a step, full / small: 74 cells of 64 x 64 71 /
     // 83, 37 of 128 x 128 102 / 93, 10 of 256 x 256 227 / 218), further up the
