@@ -316,14 +316,17 @@ int pfag_fn_saving_out_functions(pfag_ctx *ctx, void *phi_out, void *rho_out, vo
 int pfag_conv3x3(const void *x, const void *w, const float *bias, void *y, void *pre, int B, int H, int W,
                  int cin, int cout, int gelu_on, unsigned *err, void *stream);
 /* dw[co][t][ci] += sum over sites of dz[q][co] x[q + off_t][ci]; db[co] +=
- * sum of dz[q][co] (accumulates: zero dw, db first). */
+ * sum of dz[q][co] (accumulates: zero dw, db first).  dz's halo rows 0 and
+ * H+1 are not read; its halo columns must be zero. */
 int pfag_conv3x3_wgrad(const void *x, const void *dz, float *dw, float *db, int B, int H, int W, int cin,
                        int cout, unsigned *err, void *stream);
 /* dx = the input gradient of that layer from dz (BF16 [B][H+2][W+2][cout]),
  * rounded to BF16, and with gelu_on times GELU'(pre), pre the pre-activation
  * of the layer below (BF16 [B][H+2][W+2][cin]), rounded again: what
  * pfag_conv_flip, pfag_conv3x3 of dz and pfag_conv_act_bwd give, in one kernel.
- * The halo rows of dx are not written. */
+ * The halo rows of dx (rows 0 and H+1) are not written, its halo columns are
+ * zeroed: pfag_conv3x3_wgrad takes dx as it is, pfag_conv3x3 and this function
+ * read the halo rows of their input, which the caller has zeroed once. */
 int pfag_conv3x3_dgrad(const void *dz, const void *w, const void *pre, void *dx, int B, int H, int W, int cin,
                        int cout, int gelu_on, unsigned *err, void *stream);
 /* dz = dy * GELU'(pre) (gelu_on) or dy, zero on the halo. */

@@ -156,18 +156,18 @@ __device__ __forceinline__ float gelu_grad(float x) {
     return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
-// Stage pixels [q_lo, q_lo + P) of a sample (zero outside 0 .. Q-1) as
+// Stage pixels [q_lo, q_lo + P) of a sample (zero outside [lo, hi)) as
 // [C/8][ps][8]; consecutive threads take the chunks of one pixel, so a warp
 // reads whole 32-byte sectors.
 template <int C>
 __device__ __forceinline__ void stage_pixels(unsigned char *dst, int ps, const __nv_bfloat16 *__restrict__ x,
-                                             long sample_off, int q_lo, int P, int Q) {
+                                             long sample_off, int q_lo, int P, int lo, int hi) {
     constexpr int CH = C / 8;
     for (int e = threadIdx.x; e < P * CH; e += KC_THREADS) {
         const int p = e / CH, c = e - p * CH;
         const int q = q_lo + p;
         unsigned char *d = dst + ((size_t)c * ps + p) * 16;
-        if (q >= 0 && q < Q) cp16(d, x + (sample_off + q) * C + c * 8);
+        if (q >= lo && q < hi) cp16(d, x + (sample_off + q) * C + c * 8);
         else *reinterpret_cast<uint4 *>(d) = make_uint4(0, 0, 0, 0);
     }
 }
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(KC_BLOCK, 2) kc_conv_fwd(const __nv_bfloat16 *
     const auto load = [&](long tile, int st) {
         if (tile >= ntiles) return;
         const int b = (int)(tile / tiles_per), tb = (int)(tile - (long)b * tiles_per);
-        stage_pixels<CIN>(xs + st * xstage, P, x, (long)b * Q, tb * TP - 1, P, Q);   // q0 - Wp - 1, q0 = Wp + tb TP
+        stage_pixels<CIN>(xs + st * xstage, P, x, (long)b * Q, tb * TP - 1, P, 0, Q);   // q0 - Wp - 1, q0 = Wp + tb TP
     };
     const auto epilogue = [&](long tile, int acc, bool ok) {
         const int b = (int)(tile / tiles_per), tb = (int)(tile - (long)b * tiles_per);
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(KC_BLOCK, 2) kc_conv_fwd(const __nv_bfloat16 *
 }
 
 // dW[co][t][ci] += sum_q dz[q][co] x[q + off_t][ci], db[co] += sum_q dz[q][co]
-// (dz zero on halo sites).  CIN, COUT in {16, 32}; NST stages.  M = 128 holds the
+// (q over rows 1 .. H; dz zero on their halo sites).  CIN, COUT in {16, 32}; NST stages.  M = 128 holds the
 // three column shifts of a tap row: with q' = q + dx, tap (dy, dx) is
 // sum_q' dz[q' - dx][co] x[q' + dy Wp][ci], so dz is staged three times, shifted
 // by one pixel each (rows dx COUT + co), and a tile takes 3 x 8 MMAs instead of
@@ -443,10 +443,12 @@ __global__ void __launch_bounds__(KC_BLOCK) kc_conv_wgrad(const __nv_bfloat16 *_
             if (tile >= ntiles) return;
             const int b = (int)(tile / tiles_per), tb = (int)(tile - (long)b * tiles_per);
             const int q0 = Wp + tb * 128;
-            stage_pixels<CIN>(xs + st * xstage, P, x, (long)b * Q, q0 - Wp - 1, P, Q);
+            stage_pixels<CIN>(xs + st * xstage, P, x, (long)b * Q, q0 - Wp - 1, P, 0, Q);
+            // rows 1 .. H of dz only: its halo rows may hold anything
 #pragma unroll
             for (int d = 0; d < 3; d++)
-                stage_pixels<COUT>(gs + st * gstage + (size_t)d * CG * 128 * 16, 128, dz, (long)b * Q, q0 + 1 - d, 128, Q);
+                stage_pixels<COUT>(gs + st * gstage + (size_t)d * CG * 128 * 16, 128, dz, (long)b * Q, q0 + 1 - d, 128, Wp,
+                                   (H + 1) * Wp);
         };
         const auto done = [&](int kk) { return mbar_wait(smem_addr(&bar_done[kk & 1]), (kk >> 1) & 1); };
         float bsum[8];                                        // db partials: channels 8 (tid % CG) ..
