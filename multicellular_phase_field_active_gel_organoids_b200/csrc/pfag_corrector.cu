@@ -52,6 +52,7 @@ namespace {
 
 constexpr int KC_THREADS = 256;            // the warps that copy and run the epilogue
 constexpr int KC_BLOCK = KC_THREADS + 32;   // and the one that issues the MMAs
+// polls before a wait gives up (each suspends the thread for a while by itself)
 constexpr long KC_SPIN_LIMIT = 1L << 22;
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
@@ -309,6 +310,7 @@ __global__ void __launch_bounds__(KC_BLOCK, 2) kc_conv_fwd(const __nv_bfloat16 *
     int k = 0;                                                    // this CTA's stage counter
     if (threadIdx.x >= KC_THREADS) {
         // the MMA warp: stage k once it is staged and its accumulator (two, in turn) read
+        int issued = -1;                                          // the last stage whose MMAs are under way
         for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, k++) {
             const int st = NST == 2 ? k & 1 : 0;
             ok = mbar_wait(smem_addr(&bar_full[st]), NST == 2 ? (k >> 1) & 1 : k & 1);
@@ -331,8 +333,12 @@ __global__ void __launch_bounds__(KC_BLOCK, 2) kc_conv_fwd(const __nv_bfloat16 *
                 }
                 mma_commit(smem_addr(&bar_done[k & 1]));
             }
+            if (ok) issued = k;
             __syncwarp();
         }
+        // a wait elsewhere in the block that ran out may have ended it early: the
+        // last MMAs still read shared memory and write TMEM, which the block gives up
+        if (issued >= 0) ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&bar_done[issued & 1]), (issued >> 1) & 1)) && ok;
     } else {
         const auto finish = [&](long tile, int kk) {              // stage kk's epilogue, its MMAs done
             tc_fence_after();
@@ -418,6 +424,7 @@ __global__ void __launch_bounds__(KC_BLOCK) kc_conv_wgrad(const __nv_bfloat16 *_
     bool ok = true;
     int k = 0;
     if (threadIdx.x >= KC_THREADS) {
+        int issued = -1;
         for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, k++) {
             const int st = NST == 2 ? k & 1 : 0;
             ok = mbar_wait(smem_addr(&bar_full[st]), NST == 2 ? (k >> 1) & 1 : k & 1);
@@ -436,8 +443,12 @@ __global__ void __launch_bounds__(KC_BLOCK) kc_conv_wgrad(const __nv_bfloat16 *_
                                  (k == 0 && ks == 0) ? 0u : 1u);
                 mma_commit(smem_addr(&bar_done[k & 1]));
             }
+            if (ok) issued = k;
             __syncwarp();
         }
+        // a wait elsewhere in the block that ran out may have ended it early: the
+        // last MMAs still read shared memory and write TMEM, which the block gives up
+        if (issued >= 0) ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&bar_done[issued & 1]), (issued >> 1) & 1)) && ok;
     } else {
         const auto load = [&](long tile, int st) {
             if (tile >= ntiles) return;
