@@ -79,11 +79,11 @@ struct RelaxGeom {
     int cw, g, RG;  // column warps (31 zone columns each), row groups, rows per group
     int RGT;        // rows per group the kernel is built for (0: any, normals in shared memory)
 };
-// A sum as (units of 2^24, rest) of the loops' fixed-point unit, parts that a
-// warp adds as 32-bit integers (kf_relax_cells, FP32)
+// Fixed-point unit of the loops' sums (kf_relax_cells, FP32): a sum is three
+// parts of 2^40, 2^20 and 1 units, which a warp adds as 32-bit integers
 struct RelaxUnits {
-    float f24;                    // 2^24 units as a factor on the sum of |Q - P|
-    unsigned long long thr;       // the threshold in units (2^44 .. 2^45)
+    float f40;                    // the sum of |Q - P| times this is in 2^40 units
+    unsigned long long thr;       // the threshold in units (2^60 .. 2^61)
 };
 
 struct FusedRes {
@@ -2448,10 +2448,14 @@ __device__ __forceinline__ void centroid_rows(const real *__restrict__ phi, cons
 // An FP64 warp sum is ten shuffles and five FP64 additions one after another,
 // about 450 cycles, as much as the cluster barrier.  The FP32 build therefore
 // adds its threads' FP32 sums as fixed-point integers with the warp's integer
-// reduction: units of 2^-44 of the loop's threshold or finer, each sum rounded
-// to the nearest unit (a cell's total is then within 1e-12 of the threshold),
+// reduction: units of 2^-60 of the loop's threshold or finer, each sum rounded
+// to the nearest unit (exact above 2^-37 of the threshold, and elsewhere off by
+// at most 2^-61 of it, where FP64 additions round by 2^-53 of their total),
 // capped above the threshold (a NaN counts as that cap), where only the
-// comparison's outcome matters.  An FP32 sum runs over the zone rows 8k ..
+// comparison's outcome matters.  Two parts and units of 2^-44 were
+// off by some 2^-43 of the threshold, enough to end a loop an iteration early
+// or late; the third part costs the twelve-member sweep and the six cells of
+// 400 x 400 1%, smaller organoids less.  An FP32 sum runs over the zone rows 8k ..
 // 8k + 7 of one column, as in kf_resh_first and kf_relax_loops, so the three
 // take the same decisions: the FP32 blocks own whole groups of eight rows.
 // The first warp of a group leaves its rows' sum, the others (4 or 2 rows a
@@ -2475,23 +2479,31 @@ __device__ __forceinline__ float resh_inner_f(const ReshConst &k, float s, float
     return fmaf(k.a4 * (pa - pb), s, fmaf(k.a16 * tang, t, -k.b4 * (ha + hb)));
 }
 
-constexpr unsigned RELAX_CAP = 1u << 26;     // 32 lanes of this stay below 2^32; the threshold is at most 2^21
-__device__ __forceinline__ unsigned long long relax_warp_total(unsigned hi, unsigned lo) {
-    const unsigned h = __reduce_add_sync(0xffffffffu, hi), l = __reduce_add_sync(0xffffffffu, lo);
-    return ((unsigned long long)h << 24) + l;
+constexpr unsigned RELAX_CAP = 1u << 22;     // 2^40 units: above the threshold's 2^21; 32 lanes of it fit in 32 bits
+constexpr unsigned RELAX_LOW = (1u << 20) - 1;
+__device__ __forceinline__ unsigned long long relax_warp_total(unsigned hi, unsigned mid, unsigned lo) {
+    const unsigned h = __reduce_add_sync(0xffffffffu, hi), m = __reduce_add_sync(0xffffffffu, mid);
+    const unsigned l = __reduce_add_sync(0xffffffffu, lo);
+    return ((unsigned long long)min(h, RELAX_CAP) << 40) + ((unsigned long long)m << 20) + l;   // below 2^63
 }
 __device__ __forceinline__ unsigned long long relax_warp_total(unsigned long long v) {
-    return relax_warp_total((unsigned)min(v >> 24, (unsigned long long)RELAX_CAP), (unsigned)v & 0xffffffu);
+    return relax_warp_total((unsigned)(v >> 40), (unsigned)(v >> 20) & RELAX_LOW, (unsigned)v & RELAX_LOW);
 }
-__device__ __forceinline__ void relax_units_of(float f, const RelaxUnits &u, unsigned &hi, unsigned &lo) {
-    const float v = fminf(f * u.f24, (float)RELAX_CAP);       // fminf drops a NaN
+__device__ __forceinline__ void relax_units_of(float f, const RelaxUnits &u, unsigned &hi, unsigned &mid, unsigned &lo) {
+    const float v = fminf(f * u.f40, (float)RELAX_CAP);       // fminf drops a NaN
     hi = (unsigned)v;
-    lo = __float2uint_rn((v - (float)hi) * 16777216.0f);
+    const float w = (v - (float)hi) * 1048576.0f;             // exact, like the next difference
+    mid = (unsigned)w;
+    lo = __float2uint_rn((w - (float)mid) * 1048576.0f);
 }
 __device__ __forceinline__ unsigned long long relax_warp_total(float f, const RelaxUnits &u) {
-    unsigned hi, lo;
-    relax_units_of(f, u, hi, lo);
-    return relax_warp_total(hi, lo);
+    unsigned hi, mid, lo;
+    relax_units_of(f, u, hi, mid, lo);
+    return relax_warp_total(hi, mid, lo);
+}
+// sums of warp totals: either one above the cap stays above the threshold
+__device__ __forceinline__ unsigned long long relax_add(unsigned long long a, unsigned long long b) {
+    return min(a + b, (unsigned long long)RELAX_CAP << 40);
 }
 
 // Block sums of (c, sx, sy) into out[0..2] (shared), which the caller zeroed
@@ -2652,9 +2664,9 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
             if (it > 1) {
                 sum_t t;
                 if constexpr (LEAVE) {
-                    // lane sums of whole 2^24 units and rests, one warp reduction at the end
+                    // the lane's sums of the three parts, one warp reduction at the end
                     const float *d = dev + ((it - 1) & 1) * dp + lane;
-                    unsigned hi = 0, lo = 0;
+                    unsigned hi = 0, mid = 0, lo = 0;
                     for (int gr = 0; gr < gm.RC / 8; gr++, d += DR * 32 * gm.cw) {
 #pragma unroll 4
                         for (int k = 0; k < gm.cw; k++) {
@@ -2663,14 +2675,16 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
 #pragma unroll
                                 for (int r = RR; r < 8; r++) f += d[(r * gm.cw + k) * 32];
                             }
-                            unsigned h, l;
-                            relax_units_of(f, un, h, l);
+                            unsigned h, m, l;
+                            relax_units_of(f, un, h, m, l);
                             lo += l;
-                            hi = min(hi + h + (lo >> 24), RELAX_CAP);
-                            lo &= 0xffffffu;
+                            mid += m + (lo >> 20);
+                            hi = min(hi + h + (mid >> 20), RELAX_CAP);
+                            mid &= RELAX_LOW;
+                            lo &= RELAX_LOW;
                         }
                     }
-                    t = relax_warp_total(hi, lo);
+                    t = relax_warp_total(hi, mid, lo);
                 } else if constexpr (F32) t = relax_warp_total(lane < np ? wsum[((it - 1) & 1) * np + lane] : 0ull);
                 else t = warp_sum_fixed(wsum + ((it - 1) & 1) * np, np);
                 if (ptab) ptab[((it - 1) & 1) * 16 + rank] = t;
@@ -2759,13 +2773,13 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
                     for (int r = ra; r < rb; r++) {
                         row(r, (real)0.0, (real)0.0, (real)0.0, (real)0.0);
                         if constexpr (F32) {
-                            if (((r - ra) & 7) == 7) { units += relax_warp_total(facc, un); facc = 0.0f; }
+                            if (((r - ra) & 7) == 7) { units = relax_add(units, relax_warp_total(facc, un)); facc = 0.0f; }
                         }
                     }
                 }
                 if constexpr (LEAVE) {
                     if ((ra & 7) == 0) dev[(it & 1) * dp + ((ra >> 3) * DR * gm.cw + col) * 32 + lane] = facc;
-                } else if constexpr (F32) units += relax_warp_total(facc, un);
+                } else if constexpr (F32) units = relax_add(units, relax_warp_total(facc, un));
             }
             if constexpr (LEAVE) {
             } else if constexpr (F32) {
@@ -3100,13 +3114,13 @@ struct Fused {
         }
     }
     // the fixed-point unit of FP32 sums of |Q - P|: a power of two that makes the
-    // loop's threshold 2^44 .. 2^45 units; false when the threshold is no
+    // loop's threshold 2^60 .. 2^61 units; false when the threshold is no
     // positive number of usual size
     bool relax_units(RelaxUnits &u) const {
         const double t = c->dp.thr_cells / (c->dp.dx * c->dp.dx / (double)c->dp.Ncur);
         if (!(t > 1e-18 && t < 1e18)) return false;
-        const int e = 44 - std::ilogb(t);
-        u.f24 = (float)std::ldexp(1.0, e - 24);
+        const int e = 60 - std::ilogb(t);
+        u.f40 = (float)std::ldexp(1.0, e - 40);
         u.thr = (unsigned long long)std::ldexp(t, e);
         return true;
     }
