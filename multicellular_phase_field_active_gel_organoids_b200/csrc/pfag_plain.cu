@@ -246,8 +246,8 @@ __global__ void k_serial_sum_cells(const real *__restrict__ h, int N, int ncells
 
 template <typename real>
 __global__ void k_serial_absdiff(const real *__restrict__ a, const real *__restrict__ b, int N, double dx,
-                                 double *__restrict__ out) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+                                 const int *__restrict__ active, double *__restrict__ out) {
+    if (blockIdx.x != 0 || threadIdx.x != 0 || !*active) return;
     double acc = 0.0;
     for (int i = 0; i < N; i++)
         for (int j = 0; j < N; j++) {
@@ -975,7 +975,7 @@ struct Plain {
             const double *part = c->part_z;
             int npart = (int)(g.x * g.y);
             if (c->serial_sums) {
-                k_serial_absdiff<real><<<1, 32, 0, c->stream>>>(Q, R(f), N, c->dp.dx, c->d_scal + 1);
+                k_serial_absdiff<real><<<1, 32, 0, c->stream>>>(Q, R(f), N, c->dp.dx, st, c->d_scal + 1);
                 PFAG_LAUNCHED(c);
                 part = c->d_scal + 1;
                 npart = 1;
