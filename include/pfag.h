@@ -161,16 +161,19 @@ int pfag_set_lumen_tiles(pfag_ctx *ctx, int tma);
 /* ---- Batches: several organoids (fused-path contexts on the current device)
  * advanced together, the in-process form of the reference's parameter sweep
  * (main_code/setup_simulation.py:206-312 writes one folder and one batch job
- * per member).  After each member's first two steps (the first eager, the
- * second captured as its step graph) a batch step is ONE graph launch whose
- * child graphs are the members' step graphs, with no dependencies between
- * members, so the GPU runs them side by side.  Member order is the caller's
+ * per member).  After each member's first step (eager) a batch step is ONE
+ * graph launch whose child graphs are the members' steps, captured for the
+ * batch, with no dependencies between members, so the GPU runs them side by
+ * side.  Making, stepping or destroying a batch leaves the members' own step
+ * graphs as they are: a member stepped by itself before, between or after
+ * batch steps runs as if there were no batch.  Member order is the caller's
  * (group members of one box size together: the autotuner's buckets).
  * pfag_batch_step is synchronous and refreshes every member's observables
  * and statistics; pfag_batch_step_async enqueues only (the members' streams
  * wait for it, so per-member calls stay ordered after it).  A member whose
- * step graph changes (a new relaxation cap, launch shape, debug flag) makes
- * the next batch step rebuild the parent graph. */
+ * step changes (a new relaxation cap or launch shape) is captured again and
+ * the parent graph rebuilt at the next batch step; while a member has a debug
+ * flag or profiling on, the members step one by one. */
 typedef struct pfag_batch pfag_batch;
 int pfag_batch_create(pfag_ctx *const *ctxs, int n, pfag_batch **out);
 int pfag_batch_step(pfag_batch *b, int it0, int nsteps);

@@ -3,8 +3,8 @@
 The reference sweeps parameters by writing one folder and one batch job per
 member (main_code/setup_simulation.py:206-312); every member is its own
 process on its own GPU.  Here every member is a fused-path context on one
-GPU, and after two warm-up steps a step of the whole sweep is ONE graph
-launch (pfag_batch_*: the members' captured step graphs as child graphs of one
+GPU, and after one warm-up step a step of the whole sweep is ONE graph
+launch (pfag_batch_*: the members' captured steps as child graphs of one
 parent graph, no dependencies between members), so the GPU runs small
 organoids side by side instead of one after another.
 

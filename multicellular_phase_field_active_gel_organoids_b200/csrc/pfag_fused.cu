@@ -11,6 +11,8 @@ int pfag_fused_step_f64(pfag_ctx *c);
 int pfag_fused_step_f32(pfag_ctx *c);
 int pfag_fused_recentre_f64(pfag_ctx *c);
 int pfag_fused_recentre_f32(pfag_ctx *c);
+int pfag_fused_capture_f64(pfag_ctx *c, bool beside, cudaGraph_t *g, long *launches);
+int pfag_fused_capture_f32(pfag_ctx *c, bool beside, cudaGraph_t *g, long *launches);
 int pfag_fused_step_part_f64(pfag_ctx *c, int part);
 int pfag_fused_step_part_f32(pfag_ctx *c, int part);
 
@@ -82,8 +84,17 @@ extern "C" int pfag_set_lumen_tiles(pfag_ctx *c, int tma) {
 
 // ---- batches of contexts stepped as one graph ---------------------------------
 struct pfag_batch {
+    // a member's step as the batch runs it: captured for the batch, beside the
+    // member's own step graph
+    struct Child {
+        cudaGraph_t graph = nullptr;
+        long launches = 0;
+        unsigned long gen = 0;             // FusedRes::graph_gen and relaxation cap it was captured at
+        int cap = 0;
+    };
     std::vector<pfag_ctx *> m;
-    std::vector<cudaGraph_t> built_from;   // member step graphs the parent graph was built from
+    std::vector<Child> child;
+    bool refused = false;                   // a capture failed: member by member from then on
     std::vector<cudaEvent_t> mev;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev = nullptr;
@@ -98,7 +109,6 @@ static void batch_drop_graph(pfag_batch *b) {
     if (b->graph) cudaGraphDestroy(b->graph);
     b->gexec = nullptr;
     b->graph = nullptr;
-    b->built_from.clear();
 }
 
 extern "C" int pfag_batch_create(pfag_ctx *const *ctxs, int n, pfag_batch **out) {
@@ -114,6 +124,7 @@ extern "C" int pfag_batch_create(pfag_ctx *const *ctxs, int n, pfag_batch **out)
     }
     pfag_batch *b = new pfag_batch();
     b->m.assign(ctxs, ctxs + n);
+    b->child.resize(n);
     b->mev.assign(n, nullptr);
     int rc = PFAG_OK;
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -128,16 +139,6 @@ extern "C" int pfag_batch_create(pfag_ctx *const *ctxs, int n, pfag_batch **out)
         delete b;
         return rc;
     }
-    // members run side by side and fill the GPU together: each steps without
-    // the spectral passes beside its cell loops from here on (with them the
-    // twelve-member sweep took 5 to 10% longer)
-    for (pfag_ctx *c : b->m) {
-        FusedRes *r = F(c);
-        if (n == 1 || !r->split) continue;
-        r->split = false;
-        fused_drop_graph(r);
-        r->graph_state = 0;
-    }
     *out = b;
     return PFAG_OK;
 }
@@ -146,6 +147,7 @@ extern "C" int pfag_batch_destroy(pfag_batch *b) {
     if (!b) return PFAG_OK;
     if (b->stream) cudaStreamSynchronize(b->stream);
     batch_drop_graph(b);
+    for (auto &k : b->child) if (k.graph) cudaGraphDestroy(k.graph);
     for (cudaEvent_t e : b->mev) if (e) cudaEventDestroy(e);
     if (b->ev) cudaEventDestroy(b->ev);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -155,20 +157,41 @@ extern "C" int pfag_batch_destroy(pfag_batch *b) {
 
 static bool member_ready(pfag_ctx *c) {
     const FusedRes *r = F(c);
-    return r->graph_ok && !r->ring_pending;
+    return r->eager_steps >= 1 && !r->ring_pending && r->graph_state >= 0 && fused_graphable(c);
 }
 
-// the parent graph: one child node per member step graph, no edges between them
+// The parent graph: one child node per member's step, no edges between them;
+// what changed since the last build is captured again.  Members run side by
+// side and fill the GPU together, so several of them step without the spectral
+// passes beside their cell loops (with them the twelve-member sweep took 5 to
+// 10% longer).
 static int batch_build(pfag_batch *b) {
+    bool stale = !b->gexec;
+    for (size_t i = 0; i < b->m.size(); i++) {
+        pfag_ctx *c = b->m[i];
+        pfag_batch::Child &k = b->child[i];
+        if (k.graph && k.gen == F(c)->graph_gen && k.cap == c->relax_cap) continue;
+        stale = true;
+        if (k.graph) cudaGraphDestroy(k.graph);
+        k.graph = nullptr;
+        const bool alone = b->m.size() == 1;
+        const int rc = c->prec == 64 ? pfag_fused_capture_f64(c, alone, &k.graph, &k.launches)
+                                     : pfag_fused_capture_f32(c, alone, &k.graph, &k.launches);
+        if (rc != PFAG_OK) {
+            b->refused = true;
+            return PFAG_OK;
+        }
+        k.gen = F(c)->graph_gen;
+        k.cap = c->relax_cap;
+    }
+    if (!stale) return PFAG_OK;
     batch_drop_graph(b);
     PFAG_CUDA_CHECK(cudaGraphCreate(&b->graph, 0));
     b->per_step = 0;
-    for (pfag_ctx *c : b->m) {
-        FusedRes *r = F(c);
+    for (const pfag_batch::Child &k : b->child) {
         cudaGraphNode_t node;
-        PFAG_CUDA_CHECK(cudaGraphAddChildGraphNode(&node, b->graph, nullptr, 0, r->graph));
-        b->built_from.push_back(r->graph);
-        b->per_step += r->graph_launches;
+        PFAG_CUDA_CHECK(cudaGraphAddChildGraphNode(&node, b->graph, nullptr, 0, k.graph));
+        b->per_step += k.launches;
     }
     PFAG_CUDA_CHECK(cudaGraphInstantiate(&b->gexec, b->graph, 0));
     return PFAG_OK;
@@ -178,12 +201,15 @@ extern "C" int pfag_batch_step_async(pfag_batch *b, int it0, int nsteps) {
     if (!b || nsteps < 0) { pfag_set_error("pfag_batch_step: bad arguments"); return PFAG_E_ARG; }
     b->launches = 0;
     int k = 0;
-    // members step on their own streams until each has captured its step graph
-    // (the first step after an upload runs eagerly, the next one is captured)
+    // members step on their own streams until each can be captured (the first
+    // step after an upload runs eagerly)
     for (; k < nsteps; k++) {
-        bool ready = true;
+        bool ready = !b->refused;
         for (pfag_ctx *c : b->m) ready = ready && member_ready(c);
-        if (ready) break;
+        if (ready) {
+            PFAG_TRY(batch_build(b));
+            if (!b->refused) break;
+        }
         for (pfag_ctx *c : b->m) {
             const long l0 = c->launches;
             PFAG_TRY(pfag_fused_step(c, it0 + k));
@@ -191,9 +217,6 @@ extern "C" int pfag_batch_step_async(pfag_batch *b, int it0, int nsteps) {
         }
     }
     if (k == nsteps) return PFAG_OK;
-    bool stale = !b->gexec || b->built_from.size() != b->m.size();
-    for (size_t i = 0; !stale && i < b->m.size(); i++) stale = F(b->m[i])->graph != b->built_from[i];
-    if (stale) PFAG_TRY(batch_build(b));
     // the batch stream after every member's pending work, every member stream after the batch
     for (size_t i = 0; i < b->m.size(); i++) {
         PFAG_CUDA_CHECK(cudaEventRecord(b->mev[i], b->m[i]->stream));

@@ -159,6 +159,7 @@ struct FusedRes {
     int graph_state;        // 0 not tried, 1 captured, -1 capture failed (eager from then on)
     long graph_key;         // host inputs the capture depends on (relaxation cap)
     long graph_launches;    // kernel launches in one replay
+    unsigned long graph_gen;   // grows whenever what a captured step holds changes
     long eager_steps;
 };
 
@@ -2979,6 +2980,7 @@ struct Fused {
     pfag_ctx *c;
     FusedRes *r;
     cudaStream_t bs;        // the spectral passes' stream: the context's, or its own (split)
+    bool beside = true;     // false: the spectral passes on the context's stream whatever the size
     explicit Fused(pfag_ctx *ctx) : c(ctx), r(F(ctx)), bs(ctx->stream) {}
     real *R(void *p) { return (real *)p; }
 
@@ -3443,7 +3445,7 @@ struct Fused {
         // 4-5. spectral solve with the phi update after its pass A; the last
         //    column pass writes the new rho over each box in place
         //    (rho <- rhon of run_with_active_gels.cpp:175-178 on the box)
-        const bool split = fork && r->split;
+        const bool split = fork && r->split && beside;
         if (split) {
             bs = r->spec;
             PFAG_CUDA_CHECK(cudaStreamWaitEvent(bs, r->ev_psi, 0));
@@ -3761,6 +3763,7 @@ template <typename real> int fused_alloc_t(pfag_ctx *c) { return Fused<real>(c).
 template <typename real> int fused_recentre_t(pfag_ctx *c) { return Fused<real>(c).recentre(); }
 template <typename real> int fused_upload_t(pfag_ctx *c) { return Fused<real>(c).upload_hook(); }
 inline void fused_drop_graph(FusedRes *r) {
+    r->graph_gen++;
     if (r->graph_ok) { cudaGraphExecDestroy(r->gexec); cudaGraphDestroy(r->graph); }
     r->graph_ok = false;
     for (int k = 0; k < 2; k++) {
@@ -3768,6 +3771,32 @@ inline void fused_drop_graph(FusedRes *r) {
         r->pgraph_ok[k] = false;
         r->pgraph_state[k] = 0;
     }
+}
+
+// whether the context's steps may be replayed from a capture now
+inline bool fused_graphable(pfag_ctx *c) { return !pfag_prof_on(c) && !c->debug && !std::getenv("PFAG_NO_GRAPH"); }
+
+// One whole step captured as a graph (the caller's), not run; beside: as for a
+// context that steps alone.
+template <typename real> int fused_capture_t(pfag_ctx *c, bool beside, cudaGraph_t *g, long *launches) {
+    const long l0 = c->launches;
+    int rc = PFAG_E_CUDA;
+    *g = nullptr;
+    if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+        Fused<real> f(c);
+        f.beside = beside;
+        rc = f.enqueue();
+        const cudaError_t e = cudaStreamEndCapture(c->stream, g);
+        if (rc == PFAG_OK && (e != cudaSuccess || !*g)) rc = PFAG_E_CUDA;
+        if (rc != PFAG_OK && *g) {
+            cudaGraphDestroy(*g);
+            *g = nullptr;
+        }
+    }
+    *launches = c->launches - l0;
+    c->launches = l0;
+    (void)cudaGetLastError();   // a refused capture leaves a non-sticky error
+    return rc;
 }
 
 // One part of a step split at psi (part 1: head, 2: tail), graph-captured
@@ -3780,7 +3809,7 @@ template <typename real> int fused_step_part_t(pfag_ctx *c, int part) {
         return PFAG_E_ARG;
     }
     const int k = part - 1;
-    const bool graphable = !pfag_prof_on(c) && !c->debug && !std::getenv("PFAG_NO_GRAPH");
+    const bool graphable = fused_graphable(c);
     if (r->graph_key != (long)c->relax_cap) {
         fused_drop_graph(r);
         r->graph_state = 0;
@@ -3829,32 +3858,28 @@ template <typename real> int fused_step_part_t(pfag_ctx *c, int part) {
 template <typename real> int fused_step_t(pfag_ctx *c) {
     FusedRes *r = F(c);
     if (r->head_pending) { pfag_set_error("a step head is waiting for its tail"); return PFAG_E_ARG; }
-    const bool graphable = !pfag_prof_on(c) && !c->debug && !std::getenv("PFAG_NO_GRAPH");
+    const bool graphable = fused_graphable(c);
     const long key = (long)c->relax_cap;
     if (r->graph_ok && r->graph_key != key) {
         fused_drop_graph(r);
         r->graph_state = 0;
     }
     if (graphable && r->graph_state == 0 && r->eager_steps >= 1 && !r->ring_pending) {
-        cudaStream_t s = c->stream;
-        const long l0 = c->launches;
         r->graph_state = -1;
-        if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            const int rc = Fused<real>(c).enqueue();
-            cudaGraph_t g = nullptr;
-            const cudaError_t e = cudaStreamEndCapture(s, &g);
-            if (rc == PFAG_OK && e == cudaSuccess && g && cudaGraphInstantiate(&r->gexec, g, 0) == cudaSuccess) {
+        cudaGraph_t g = nullptr;
+        long launches = 0;
+        if (fused_capture_t<real>(c, true, &g, &launches) == PFAG_OK) {
+            if (cudaGraphInstantiate(&r->gexec, g, 0) == cudaSuccess) {
                 r->graph = g;
                 r->graph_ok = true;
                 r->graph_state = 1;
                 r->graph_key = key;
-                r->graph_launches = c->launches - l0;
-            } else if (g) {
+                r->graph_launches = launches;
+            } else {
                 cudaGraphDestroy(g);
+                (void)cudaGetLastError();
             }
         }
-        c->launches = l0;
-        (void)cudaGetLastError();   // a refused capture leaves a non-sticky error
     }
     int rc = PFAG_OK;
     if (r->graph_ok && !r->ring_pending && graphable) {
