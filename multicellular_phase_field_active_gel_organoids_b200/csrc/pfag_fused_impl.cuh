@@ -79,11 +79,10 @@ struct RelaxGeom {
     int cw, g, RG;  // column warps (31 zone columns each), row groups, rows per group
     int RGT;        // rows per group the kernel is built for (0: any, normals in shared memory)
 };
-// Fixed-point unit of the loops' sums (kf_relax_cells, FP32): a sum is three
-// parts of 2^40, 2^20 and 1 units, which a warp adds as 32-bit integers
+// Fixed-point unit of the loops' sums (kf_relax_cells, FP32)
 struct RelaxUnits {
-    float f40;                    // the sum of |Q - P| times this is in 2^40 units
-    unsigned long long thr;       // the threshold in units (2^60 .. 2^61)
+    float scale;                  // a sum of |Q - P| times this is in units
+    unsigned long long thr;       // the threshold in units (2^57 .. 2^58)
 };
 
 struct FusedRes {
@@ -2448,15 +2447,14 @@ __device__ __forceinline__ void centroid_rows(const real *__restrict__ phi, cons
 // are kept: with it the last, phi is iterate it - 1.
 // An FP64 warp sum is ten shuffles and five FP64 additions one after another,
 // about 450 cycles, as much as the cluster barrier.  The FP32 build therefore
-// adds its threads' FP32 sums as fixed-point integers with the warp's integer
-// reduction: units of 2^-60 of the loop's threshold or finer, each sum rounded
-// to the nearest unit (exact above 2^-37 of the threshold, and elsewhere off by
-// at most 2^-61 of it, where FP64 additions round by 2^-53 of their total),
-// capped above the threshold (a NaN counts as that cap), where only the
-// comparison's outcome matters.  Two parts and units of 2^-44 were
-// off by some 2^-43 of the threshold, enough to end a loop an iteration early
-// or late; the third part costs the twelve-member sweep and the six cells of
-// 400 x 400 1%, smaller organoids less.  An FP32 sum runs over the zone rows 8k ..
+// adds its threads' FP32 sums as fixed-point numbers, in three 32-bit parts by
+// the warp's integer reduction: units of 2^-57 of the loop's threshold or
+// finer, each sum rounded to the nearest unit (exact above 2^-33 of the
+// threshold, and elsewhere off by at most 2^-58 of it, where FP64 additions
+// round by 2^-53 of their total), capped above the threshold (a NaN counts as
+// that cap), where only the comparison's outcome matters.  Two parts and units
+// of 2^-44 were off by some 2^-43 of the threshold, enough to end a loop an
+// iteration early or late.  An FP32 sum runs over the zone rows 8k ..
 // 8k + 7 of one column, as in kf_resh_first and kf_relax_loops, so the three
 // take the same decisions: the FP32 blocks own whole groups of eight rows.
 // The first warp of a group leaves its rows' sum, the others (4 or 2 rows a
@@ -2480,31 +2478,17 @@ __device__ __forceinline__ float resh_inner_f(const ReshConst &k, float s, float
     return fmaf(k.a4 * (pa - pb), s, fmaf(k.a16 * tang, t, -k.b4 * (ha + hb)));
 }
 
-constexpr unsigned RELAX_CAP = 1u << 22;     // 2^40 units: above the threshold's 2^21; 32 lanes of it fit in 32 bits
-constexpr unsigned RELAX_LOW = (1u << 20) - 1;
-__device__ __forceinline__ unsigned long long relax_warp_total(unsigned hi, unsigned mid, unsigned lo) {
-    const unsigned h = __reduce_add_sync(0xffffffffu, hi), m = __reduce_add_sync(0xffffffffu, mid);
-    const unsigned l = __reduce_add_sync(0xffffffffu, lo);
-    return ((unsigned long long)min(h, RELAX_CAP) << 40) + ((unsigned long long)m << 20) + l;   // below 2^63
+constexpr unsigned long long RELAX_CAP = 1ull << 59;          // above the threshold's 2^58
+__device__ __forceinline__ unsigned long long relax_units_of(float f, const RelaxUnits &u) {
+    return __float2ull_rn(fminf(f * u.scale, (float)RELAX_CAP));   // fminf drops a NaN
 }
+// sum over the warp of values below 2^63: exact, or capped at about 2 RELAX_CAP
 __device__ __forceinline__ unsigned long long relax_warp_total(unsigned long long v) {
-    return relax_warp_total((unsigned)(v >> 40), (unsigned)(v >> 20) & RELAX_LOW, (unsigned)v & RELAX_LOW);
-}
-__device__ __forceinline__ void relax_units_of(float f, const RelaxUnits &u, unsigned &hi, unsigned &mid, unsigned &lo) {
-    const float v = fminf(f * u.f40, (float)RELAX_CAP);       // fminf drops a NaN
-    hi = (unsigned)v;
-    const float w = (v - (float)hi) * 1048576.0f;             // exact, like the next difference
-    mid = (unsigned)w;
-    lo = __float2uint_rn((w - (float)mid) * 1048576.0f);
-}
-__device__ __forceinline__ unsigned long long relax_warp_total(float f, const RelaxUnits &u) {
-    unsigned hi, mid, lo;
-    relax_units_of(f, u, hi, mid, lo);
-    return relax_warp_total(hi, mid, lo);
-}
-// sums of warp totals: either one above the cap stays above the threshold
-__device__ __forceinline__ unsigned long long relax_add(unsigned long long a, unsigned long long b) {
-    return min(a + b, (unsigned long long)RELAX_CAP << 40);
+    constexpr unsigned LOW = (1u << 20) - 1;
+    const unsigned h = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 40));
+    const unsigned m = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 20) & LOW);
+    const unsigned l = __reduce_add_sync(0xffffffffu, (unsigned)v & LOW);
+    return ((unsigned long long)min(h, (unsigned)(RELAX_CAP >> 39)) << 40) + ((unsigned long long)m << 20) + l;
 }
 
 // Block sums of (c, sx, sy) into out[0..2] (shared), which the caller zeroed
@@ -2665,9 +2649,10 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
             if (it > 1) {
                 sum_t t;
                 if constexpr (LEAVE) {
-                    // the lane's sums of the three parts, one warp reduction at the end
+                    // the lane's sum of at most 15 values (RGT = 8: a block of 16 warps; else RC = 8
+                    // and at most 10 warps a row group), one warp reduction at the end
                     const float *d = dev + ((it - 1) & 1) * dp + lane;
-                    unsigned hi = 0, mid = 0, lo = 0;
+                    unsigned long long v = 0;
                     for (int gr = 0; gr < gm.RC / 8; gr++, d += DR * 32 * gm.cw) {
 #pragma unroll 4
                         for (int k = 0; k < gm.cw; k++) {
@@ -2676,16 +2661,10 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
 #pragma unroll
                                 for (int r = RR; r < 8; r++) f += d[(r * gm.cw + k) * 32];
                             }
-                            unsigned h, m, l;
-                            relax_units_of(f, un, h, m, l);
-                            lo += l;
-                            mid += m + (lo >> 20);
-                            hi = min(hi + h + (mid >> 20), RELAX_CAP);
-                            mid &= RELAX_LOW;
-                            lo &= RELAX_LOW;
+                            v += relax_units_of(f, un);
                         }
                     }
-                    t = relax_warp_total(hi, mid, lo);
+                    t = relax_warp_total(v);
                 } else if constexpr (F32) t = relax_warp_total(lane < np ? wsum[((it - 1) & 1) * np + lane] : 0ull);
                 else t = warp_sum_fixed(wsum + ((it - 1) & 1) * np, np);
                 if (ptab) ptab[((it - 1) & 1) * 16 + rank] = t;
@@ -2770,17 +2749,16 @@ __global__ void __launch_bounds__(RelaxMax<real, RGT>::THREADS) kf_relax_cells(r
                     for (int k = 0; k < RR; k++)
                         if (ra + k < rb) row(ra + k, xs[k + 1], xt[k + 1], ys[k], yt[k]);   // warp-uniform
                 } else {
+                    for (int r8 = ra; r8 < rb; r8 += 8) {
+                        const int re = min(r8 + 8, rb);
 #pragma unroll 2
-                    for (int r = ra; r < rb; r++) {
-                        row(r, (real)0.0, (real)0.0, (real)0.0, (real)0.0);
-                        if constexpr (F32) {
-                            if (((r - ra) & 7) == 7) { units = relax_add(units, relax_warp_total(facc, un)); facc = 0.0f; }
-                        }
+                        for (int r = r8; r < re; r++) row(r, (real)0.0, (real)0.0, (real)0.0, (real)0.0);
+                        if constexpr (F32) { units = min(units + relax_units_of(facc, un), RELAX_CAP); facc = 0.0f; }
                     }
                 }
                 if constexpr (LEAVE) {
                     if ((ra & 7) == 0) dev[(it & 1) * dp + ((ra >> 3) * DR * gm.cw + col) * 32 + lane] = facc;
-                } else if constexpr (F32) units = relax_add(units, relax_warp_total(facc, un));
+                } else if constexpr (F32) units = relax_warp_total(units);
             }
             if constexpr (LEAVE) {
             } else if constexpr (F32) {
@@ -3116,13 +3094,13 @@ struct Fused {
         }
     }
     // the fixed-point unit of FP32 sums of |Q - P|: a power of two that makes the
-    // loop's threshold 2^60 .. 2^61 units; false when the threshold is no
+    // loop's threshold 2^57 .. 2^58 units; false when the threshold is no
     // positive number of usual size
     bool relax_units(RelaxUnits &u) const {
         const double t = c->dp.thr_cells / (c->dp.dx * c->dp.dx / (double)c->dp.Ncur);
         if (!(t > 1e-18 && t < 1e18)) return false;
-        const int e = 60 - std::ilogb(t);
-        u.f40 = (float)std::ldexp(1.0, e - 40);
+        const int e = 57 - std::ilogb(t);
+        u.scale = (float)std::ldexp(1.0, e);
         u.thr = (unsigned long long)std::ldexp(t, e);
         return true;
     }
