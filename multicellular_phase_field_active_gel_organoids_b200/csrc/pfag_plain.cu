@@ -266,12 +266,22 @@ __global__ void k_serial_cell_rdev(const real *__restrict__ pn, const real *__re
     if (n >= ncells) return;
     double acc = 0.0;
     if (active[n])
-        for (int i = xc[n] - z; i < xc[n] + z; i++)
-            for (int j = yc[n] - z; j < yc[n] + z; j++) {
-                const size_t o = cidx(n, i, j, N);
-                const size_t t = compact ? cidx(n, i - xc[n] + z, j - yc[n] + z, 2 * z) : o;   // [Ntot][2z][2z]
-                acc += fabs((double)pn[t] - (double)p[o]) * dx * dx / ncur;
+        for (int i = 0; i < 2 * z; i++) {
+            const real *a = p + cidx(n, xc[n] - z + i, yc[n] - z, N);
+            const real *b = compact ? pn + cidx(n, i, 0, 2 * z) : pn + (a - p);                 // [Ntot][2z][2z]
+            // eight loads of each before their additions, which wait for one another (a step
+            // of seven cells on 256^2 106 -> 83 ms)
+            for (int j0 = 0; j0 < 2 * z; j0 += 8) {
+                const int m = min(8, 2 * z - j0);
+                real u[8], v[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (k < m) { u[k] = a[j0 + k]; v[k] = b[j0 + k]; }
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (k < m) acc += fabs((double)v[k] - (double)u[k]) * dx * dx / ncur;
             }
+        }
     out[n] = acc;
 }
 
