@@ -3127,11 +3127,12 @@ struct Fused {
         } else {
             cudaLaunchAttribute attr[1];
             const cudaLaunchConfig_t cfg = relax_config(gm, smem, attr, nullptr);
-            if (cudaOccupancyMaxActiveClusters(&ncl, fn, &cfg) != cudaSuccess) {
-                (void)cudaGetLastError();
+            if (cudaOccupancyMaxActiveClusters(&ncl, fn, &cfg) == cudaSuccess) {
+                known[key] = ncl;
+            } else {
+                (void)cudaGetLastError();      // not for this context; the next one asks again
                 ncl = 0;
             }
-            known[key] = ncl;
         }
         *fits = ncl >= c->Ntot;
         return PFAG_OK;
