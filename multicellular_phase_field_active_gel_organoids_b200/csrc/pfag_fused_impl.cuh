@@ -77,7 +77,7 @@ struct RelaxGeom {
     int C;          // blocks per cluster (1: a block barrier instead of the cluster's)
     int RC;         // zone rows per block
     int cw, g, RG;  // column warps (31 zone columns each), row groups, rows per group
-    int RGT;        // rows per group the kernel is built for (0: any, normals in shared memory)
+    int RGT;        // rows per group the kernel is built for (0: any, the normals read in every iteration)
 };
 // Fixed-point unit of the loops' sums (kf_relax_cells, FP32)
 struct RelaxUnits {
@@ -3145,17 +3145,23 @@ struct Fused {
     // of 258 x 258 at 2 to 3 iterations took 437 us a step against 356 with
     // iteration 1 at full occupancy and the persistent kernel, which organoids
     // with that many cells keep.  Within a size the most row groups that stay
-    // resident.  The form that reads the normals again, where registers could
-    // hold them in a larger block, only up to 2.5 blocks per SM: 64 cells of 130
-    // x 130 at one iteration took 78 us so, 25 with iteration 1 at full occupancy
-    // and the persistent kernel; the sweep's members of 29 to 37 such cells gain
-    // (twelve members 3.38 -> 2.96 ms for four steps).
+    // resident.  The form that reads the normals again, after the largest block of
+    // the size, only up to 2.5 blocks per SM: 64 cells of 130 x 130 at one
+    // iteration took 78 us so, 25 with iteration 1 at full occupancy and the
+    // persistent kernel; the sweep's members of 29 to 37 such cells gain (twelve
+    // members 3.38 -> 2.96 ms for four steps).  Up to there it does not lose where
+    // the loops end after one iteration and gains beyond (us a step, clusters /
+    // persistent kernel, FP32 130 x 130: 17 cells 82 / 83 at one iteration, 86 /
+    // 114 at 3; 29 cells 84 / 91, 140 / 270 at 11; 41 cells 108 / 109, 131 / 231
+    // at 8; 60 cells 127 / 130, 143 / 196 at 5).  Beyond 2.5 blocks per SM it
+    // loses up to 4% at one iteration and gains at ten (53 cells of 180 x 180
+    // 268 / 259, 330 / 491): the loops of a developed organoid end after one to three.
     int choose_clusters(int nsm) {
         r->clusters = false;
         if (sizeof(real) == 4 && !relax_units(r->ru)) return PFAG_OK;
         constexpr bool F32 = sizeof(real) == 4;
         for (int C = 16; C >= 8; C /= 2) {
-            bool regs = false;     // some form keeps the normals in registers
+            bool first = true;     // no block of this size yet
             for (int k = 1; k <= 128; k++) {
                 // FP32: 2, 4, 8 rows a warp in registers, then 8, 16, ... without;
                 // FP64: 1 .. 4, then 5, 6, ...
@@ -3165,9 +3171,9 @@ struct Fused {
                 size_t smem = 0;
                 bool fits = false;
                 if (!relax_geom(C, RG, RGT, gm, smem)) continue;
-                if (RGT == 0 && regs && 2L * c->Ntot * gm.C > 5L * nsm) break;
+                if (RGT == 0 && !first && 2L * c->Ntot * gm.C > 5L * nsm) break;
                 if (RGT == 0 && gm.g == 1 && RG > gm.RC) break;
-                regs = true;
+                first = false;
                 PFAG_TRY(relax_resident(gm, smem, nsm, &fits));
                 if (fits) {
                     r->rg = gm;
