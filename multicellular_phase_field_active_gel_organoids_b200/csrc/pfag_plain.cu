@@ -5,6 +5,7 @@
 #include "pfag_internal.cuh"
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 
 namespace {
 
@@ -1170,10 +1171,10 @@ struct Plain {
     // One stretch of the step without a look of the host: enqueued by f, and from
     // the second step on replayed as a CUDA graph (about 100 launches of a step
     // in five graphs: 7 cells of 130 x 130, 693 us a step with single launches,
-    // 474 so).
+    // 474 so).  Profiling and PFAG_NO_GRAPH keep the single launches.
     template <typename Fn> int stretch(int k, Fn f) {
         PlainGraphs *pg = (PlainGraphs *)c->plain_graphs;
-        if (!pg || pg->steps < 1 || pg->failed || pfag_prof_on(c)) return f();
+        if (!pg || pg->steps < 1 || pg->failed || pfag_prof_on(c) || std::getenv("PFAG_NO_GRAPH")) return f();
         if (!pg->exec[k]) {
             const long l0 = c->launches;
             pg->failed = true;
