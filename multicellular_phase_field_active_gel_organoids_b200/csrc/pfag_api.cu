@@ -87,7 +87,7 @@ static void free_ctx(pfag_ctx *c) {
                     c->hecm, c->psi, c->d_xc, c->d_yc, c->d_cacc, c->d_s, c->d_f0, c->d_part, c->d_scal,
                     c->d_iflags, c->d_err, c->d_vx, c->d_vy};
     for (void *b : bufs) if (b) cudaFree(b);
-    void *hb[] = {c->h_iflags, c->h_scal, c->h_err, c->h_rep};
+    void *hb[] = {c->h_iflags, c->h_err, c->h_rep};
     for (void *b : hb) if (b) cudaFreeHost(b);
     delete[] c->h_xc; delete[] c->h_yc; delete[] c->h_s; delete[] c->h_f0;
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -141,7 +141,6 @@ extern "C" int pfag_create(const pfag_params *p, int precision, int path, pfag_c
         cudaMemset(c->d_err, 0, sizeof(unsigned) * 4);
         cudaMemset(c->d_scal, 0, sizeof(double) * 64);
         if (cudaMallocHost((void **)&c->h_iflags, sizeof(int) * (8 * c->Ntot + 64)) != cudaSuccess ||
-            cudaMallocHost((void **)&c->h_scal, sizeof(double) * 64) != cudaSuccess ||
             cudaMallocHost((void **)&c->h_err, sizeof(unsigned) * 4) != cudaSuccess ||
             cudaHostAlloc(&c->h_rep, report_bytes(c->Ntot), cudaHostAllocMapped) != cudaSuccess) {
             pfag_set_error("pinned host allocation failed");

@@ -105,7 +105,6 @@ struct pfag_ctx {
     int *h_xc, *h_yc;
     double *h_s, *h_f0;
     int *h_iflags;        // pinned
-    double *h_scal;       // pinned
     unsigned *h_err;      // pinned
     void *h_rep;          // pinned, mapped: what a synchronising call reads back (pfag_finish)
     pfag_stats stats;

@@ -1,7 +1,8 @@
 """pfag_conv3x3_wgrad does not read the halo rows of dz: with NaN there the
 gradients match the float64 oracle as with zeros (bounds of test_gpu_conv.py),
 on one tile, ragged last tiles, the one-stage form and on a dx that
-pfag_conv3x3_dgrad wrote into a buffer nobody zeroed."""
+pfag_conv3x3_dgrad wrote into a buffer nobody zeroed.  And the widths at which
+the kernels go from two stages to one."""
 import numpy as np
 import pytest
 
@@ -9,6 +10,7 @@ torch = pytest.importorskip("torch")
 
 from multicellular_phase_field_active_gel_organoids_b200 import capi  # noqa: E402
 from oracle import conv_oracle as co  # noqa: E402
+from tests import test_gpu_conv_staged as staged  # noqa: E402
 from tests.test_gpu_conv import P, dev  # noqa: E402
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +63,12 @@ def test_weight_gradient_of_an_input_gradient_in_a_fresh_buffer():
     rdw, rdb = co.conv_wgrad(x.float().cpu().numpy(), inner)
     assert np.max(np.abs(dw - rdw)) <= 1e-3 * np.abs(rdw).max()
     assert np.max(np.abs(db - rdb)) <= 1e-3 * np.abs(rdb).max()
+
+
+@pytest.mark.parametrize("W,cin,cout", [(477, 32, 16), (478, 32, 16), (597, 32, 32), (598, 32, 32), (633, 32, 16),
+                                        (634, 32, 16), (1021, 16, 32), (1022, 16, 32), (1397, 16, 32), (1398, 16, 32),
+                                        (1433, 16, 16), (1434, 16, 16)])
+def test_widths_beside_the_change_of_stages(W, cin, cout):
+    """The widest boxes of the two-stage forms and the narrowest of the one-stage
+    ones (weight gradient 477 and 1021, forward the others)."""
+    staged.test_forward_and_weight_gradient(1, 2, W, cin, cout)
