@@ -5,12 +5,18 @@ fixture script and bench.py's CPU baseline leg, never by the product.
 The library holds the reference's globals, so one process serves one
 configuration; `run_reference()` therefore runs in a fresh subprocess by
 default.
+
+Where the reference build is absent (its sources are not on the machine), the C
+restatement of the same step (oracle/port.py) runs instead and says so on
+stderr: tests/test_oracle.py holds it to states that the reference's own build
+wrote (tests/golden), bit for bit.
 """
 from __future__ import annotations
 
 import ctypes
 import multiprocessing as mp
 import os
+import sys
 
 import numpy as np
 
@@ -99,9 +105,43 @@ class RefLib:
         }
 
 
+class PortRun:
+    """The restatement with the calls of RefLib that a run needs."""
+
+    def __init__(self, precision: str, params: dict):
+        from oracle import port
+        self.p = port.Port(params, 64 if precision == "fp64" else 32)
+        self.M = 2 * int(params["zone_size"]) - 2
+
+    def load(self, phi, rho, lum, ecm):
+        self.p.load(phi, rho, lum, ecm)
+
+    def step(self, it: int):
+        self.p.step(it)
+
+    def step_with_velocity(self, it: int):
+        """As RefLib.step_with_velocity: the restatement's transforms run in the
+        same shim, in the same order (per cell: vx, vy, rho)."""
+        L, n, M = self.p.lib, self.p.ncells, self.M
+        buf = np.zeros(3 * n * M * M, dtype=np.float64)
+        L.pfag_shim_capture.argtypes = [ctypes.c_void_p, ctypes.c_long]
+        L.pfag_shim_capture_len.restype = ctypes.c_long
+        L.pfag_shim_capture(buf.ctypes.data_as(ctypes.c_void_p), buf.size)
+        self.step(it)
+        got = L.pfag_shim_capture_len()
+        L.pfag_shim_capture(None, 0)
+        if got != buf.size:
+            raise RuntimeError(f"captured {got} values, expected {buf.size}")
+        v = buf.reshape(n, 3, M, M) / float(M * M)
+        return v[:, 0].copy(), v[:, 1].copy()
+
+    def state(self):
+        return self.p.state()
+
+
 def _worker(precision, params, init, nsteps, start_it, extra, velocity, q):
     try:
-        r = RefLib(precision, params)
+        r = (RefLib if available(precision) else PortRun)(precision, params)
         r.load(*init)
         out_steps = {}
         vel = None
@@ -125,6 +165,8 @@ def run_reference(params: dict, init, nsteps: int, precision: str = "fp64", star
     """Run `nsteps` reference steps from `init` = (phi, rho, lum, ECM) in a
     spawned subprocess and return the final state dict (plus snapshots, and the
     last step's per-cell velocity when `velocity` is set)."""
+    if not available(precision):
+        print(f"oracle: no reference build ({lib_path(precision)}); the C restatement runs instead", file=sys.stderr)
     ctx = mp.get_context("spawn")
     q = ctx.Queue()
     p = ctx.Process(target=_worker, args=(precision, params, init, nsteps, start_it,
